@@ -693,7 +693,9 @@ PauliTerms prepare_terms(const uint64_t* xm, const uint64_t* zm, const double* c
 template <typename T>
 void transition(const vec2_t<T>* bra, const vec2_t<T>* ket, int n, const PauliTerms& terms,
                 cudaStream_t st, Workspace& ws, double out[2]) {
-    if (terms.gx.empty()) { out[0] = out[1] = 0; return; }
+    out[0] = out[1] = 0;
+    if (terms.gx.empty()) return;
+    if (bra == ket && pauli_energy<T>(ket, n, terms, st, ws, out)) return;
     const uint64_t dim = 1ull << n;
     TermPtrs tp = upload_terms(terms, st, ws);
     const unsigned nb = red_blocks(dim);

@@ -235,6 +235,10 @@ template <typename T>
 void transition(const vec2_t<T>* bra, const vec2_t<T>* ket, int n, const PauliTerms& terms,
                 cudaStream_t st, Workspace& ws, double out[2]);
 
+// <psi|H|psi> for real coefficients and n >= 12 (kern_pauli.cu); false, having done nothing, otherwise.
+template <typename T>
+bool pauli_energy(const vec2_t<T>* psi, int n, const PauliTerms& terms, cudaStream_t st, Workspace& ws, double* out);
+
 // out = H psi (gather form, no atomics)
 template <typename T>
 void apply_observable(const vec2_t<T>* psi, vec2_t<T>* out, int n, const PauliTerms& terms,
