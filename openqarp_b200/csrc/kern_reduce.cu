@@ -15,6 +15,7 @@
 #include <numeric>
 
 #include "kernels.h"
+#include "traj_rng.cuh"
 
 namespace qsv {
 
@@ -441,6 +442,53 @@ __device__ __forceinline__ double prob(const vec2_t<T>& a) {
                      __dmul_rn(static_cast<double>(a.y), static_cast<double>(a.y)));
 }
 
+// The uniforms of n shots from one engine: u[s] as std::generate_canonical<double, 53> draws them from
+// std::mt19937(seed), two outputs a shot (traj_rng.cuh states the generator).  One block: a twist is
+// three parallel steps (word k needs the new word k - 227), its 624 outputs make 312 uniforms.
+__device__ void mt_uniforms(uint32_t seed, double* __restrict__ u, size_t n) {
+    __shared__ uint32_t mt[2][kMtN];
+    const int t = threadIdx.x;
+    if (t == 0) {
+        uint32_t x = seed;
+        mt[0][0] = x;
+        for (int i = 1; i < kMtN; ++i) {
+            x = 1812433253u * (x ^ (x >> 30)) + static_cast<uint32_t>(i);
+            mt[0][i] = x;
+        }
+    }
+    __syncthreads();
+    constexpr int kStep = kMtN - kMtM;   // 227
+    static_assert(kChunkThreads == kRed && kStep <= kRed && kMtN - 2 * kStep <= kRed, "a step's words fit the block");
+    auto mixed = [](uint32_t hi, uint32_t lo) {
+        const uint32_t y = (hi & 0x80000000u) | (lo & 0x7fffffffu);
+        return (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
+    };
+    auto temper = [](uint32_t y) {
+        y ^= y >> 11;
+        y ^= (y << 7) & 0x9d2c5680u;
+        y ^= (y << 15) & 0xefc60000u;
+        return y ^ (y >> 18);
+    };
+    int cur = 0;
+    for (size_t at = 0; at < n; at += kMtN / 2) {
+        const uint32_t* o = mt[cur];
+        uint32_t* w = mt[cur ^ 1];
+        if (t < kStep) w[t] = o[t + kMtM] ^ mixed(o[t], o[t + 1]);
+        __syncthreads();
+        if (t < kStep) w[kStep + t] = w[t] ^ mixed(o[kStep + t], o[kStep + t + 1]);
+        __syncthreads();
+        const int k = 2 * kStep + t;
+        if (k < kMtN) w[k] = w[k - kStep] ^ mixed(o[k], k + 1 < kMtN ? o[k + 1] : w[0]);
+        __syncthreads();
+        for (int j = t; j < kMtN / 2 && at + j < n; j += kRed) {
+            const uint64_t v = temper(w[2 * j]) | (static_cast<uint64_t>(temper(w[2 * j + 1])) << 32);
+            const double d = __ull2double_rn(v) * 0x1p-64;
+            *QSV_DBG(u + (at + j)) = d >= 1.0 ? 0x1.fffffffffffffp-1 : d;
+        }
+        cur ^= 1;
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kRed) k_prob_total(const vec2_t<T>* __restrict__ s, uint64_t dim, double2* __restrict__ partials) {
     double2 acc = make_double2(0, 0);
@@ -451,49 +499,55 @@ __global__ void __launch_bounds__(kRed) k_prob_total(const vec2_t<T>* __restrict
     if (threadIdx.x == 0) *QSV_DBG(partials + blockIdx.x) = acc;
 }
 
-// in-chunk inclusive scan of p_i / S: thread t owns amplitudes [t*16, t*16+16) of the chunk.
-// Returns the thread's running values in `v` and writes the block total to *total.
+// One chunk's inclusive scan of p_i / S in the sampler's fixed order: thread t sums amplitudes
+// [16 t, 16 t + 16) left to right, the thread sums are added left to right, and element r of thread t
+// is base_t + run_r.  Written are the chunk's sum and base_t of every 16th thread (kGroups a chunk,
+// 1/512 of the register); k_sample_shots rebuilds the 16 threads' part around a shot from those.
+// The amplitudes are read in order and turned through shared memory: 234 us at 26 qubits; each thread
+// reading its own 16 took 288.
+// Where first is 1, block 0 draws the shots' uniforms instead: the engine is one serial chain (243 us
+// for 100 000 shots) and runs beside the other blocks' read of the register.
+constexpr int kGroups = kChunkThreads / kPerThread;   // 16
 template <typename T>
-__device__ void chunk_scan(const vec2_t<T>* __restrict__ s, uint64_t start, uint64_t dim, double inv_total_unused,
-                           double total, double v[kPerThread], double* sh, double* block_total) {
-    (void)inv_total_unused;
+__global__ void __launch_bounds__(kChunkThreads) k_chunk_totals(const vec2_t<T>* __restrict__ s, uint64_t dim,
+                                                                const double2* __restrict__ total_p,
+                                                                double* __restrict__ chunk_total, double* __restrict__ bases,
+                                                                unsigned first, uint32_t seed, double* __restrict__ u,
+                                                                size_t n_shots) {
+    if (blockIdx.x < first) {
+        mt_uniforms(seed, u, n_shots);
+        return;
+    }
+    const unsigned chunk = blockIdx.x - first;
+    __shared__ double q[(1 << kChunkLog) + kChunkThreads];   // 16 values and a pad word per thread
+    __shared__ double sh[kChunkThreads];
     const int t = threadIdx.x;
-    double run = 0;
+    const uint64_t start = static_cast<uint64_t>(chunk) << kChunkLog;
+    const double total = QSV_DBG(total_p)->x;
 #pragma unroll
     for (int r = 0; r < kPerThread; ++r) {
-        const uint64_t i = start + static_cast<uint64_t>(t) * kPerThread + r;
-        const double q = i < dim ? __ddiv_rn(prob<T>(*QSV_DBG(s + i)), total) : 0.0;
-        run = __dadd_rn(run, q);
-        v[r] = run;
+        const int j = r * kChunkThreads + t;
+        q[j + j / kPerThread] = start + j < dim ? __ddiv_rn(prob<T>(*QSV_DBG(s + (start + j))), total) : 0.0;
     }
-    // exclusive scan of thread totals, in thread order (sequential per warp lane 0 of warp 0)
+    __syncthreads();
+    double run = 0;
+#pragma unroll
+    for (int r = 0; r < kPerThread; ++r) run = __dadd_rn(run, q[t * (kPerThread + 1) + r]);
     sh[t] = run;
     __syncthreads();
     if (t == 0) {
         double acc = 0;
-        for (int u = 0; u < kChunkThreads; ++u) {
-            const double x = sh[u];
-            sh[u] = acc;
-            acc = __dadd_rn(acc, x);
-        }
-        *block_total = acc;
-    }
-    __syncthreads();
-    const double base = sh[t];
+#pragma unroll 1
+        for (int g = 0; g < kGroups; ++g) {
+            double x[kPerThread];
 #pragma unroll
-    for (int r = 0; r < kPerThread; ++r) v[r] = __dadd_rn(base, v[r]);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kChunkThreads) k_chunk_totals(const vec2_t<T>* __restrict__ s, uint64_t dim,
-                                                                const double2* __restrict__ total_p,
-                                                                double* __restrict__ chunk_total) {
-    __shared__ double sh[kChunkThreads];
-    __shared__ double tot;
-    double v[kPerThread];
-    const uint64_t start = static_cast<uint64_t>(blockIdx.x) << kChunkLog;
-    chunk_scan<T>(s, start, dim, 0.0, QSV_DBG(total_p)->x, v, sh, &tot);
-    if (threadIdx.x == 0) *QSV_DBG(chunk_total + blockIdx.x) = tot;
+            for (int k = 0; k < kPerThread; ++k) x[k] = sh[g * kPerThread + k];
+            *QSV_DBG(bases + (static_cast<uint64_t>(chunk) * kGroups + g)) = acc;
+#pragma unroll
+            for (int k = 0; k < kPerThread; ++k) acc = __dadd_rn(acc, x[k]);
+        }
+        *QSV_DBG(chunk_total + chunk) = acc;
+    }
 }
 
 // exclusive prefix of the chunk totals, off[c] = sum_{c' < c}, in a fixed order: thread t sums
@@ -507,20 +561,27 @@ __global__ void __launch_bounds__(kOffThreads) k_chunk_offsets(const double* __r
     const unsigned per = (n_chunks + kOffThreads - 1) / kOffThreads;
     const unsigned c0 = min(n_chunks, threadIdx.x * per), c1 = min(n_chunks, c0 + per);
     double acc = 0;
+#pragma unroll 8
     for (unsigned c = c0; c < c1; ++c) acc = __dadd_rn(acc, *QSV_DBG(chunk_total + c));
     run_base[threadIdx.x] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
         double a = 0;
-        for (int t = 0; t < kOffThreads; ++t) {
-            const double x = run_base[t];
-            run_base[t] = a;
-            a = __dadd_rn(a, x);
+        for (int t = 0; t < kOffThreads; t += 16) {
+            double x[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) x[k] = run_base[t + k];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                run_base[t + k] = a;
+                a = __dadd_rn(a, x[k]);
+            }
         }
         run_base[kOffThreads] = a;
     }
     __syncthreads();
     double a = run_base[threadIdx.x];
+#pragma unroll 8
     for (unsigned c = c0; c < c1; ++c) {
         *QSV_DBG(off + c) = a;
         a = __dadd_rn(a, *QSV_DBG(chunk_total + c));
@@ -528,47 +589,70 @@ __global__ void __launch_bounds__(kOffThreads) k_chunk_offsets(const double* __r
     if (threadIdx.x == 0) *QSV_DBG(off + n_chunks) = run_base[kOffThreads];
 }
 
-__device__ __forceinline__ size_t first_greater(const double* u, size_t n, double x) {
-    size_t lo = 0, hi = n;   // first s with u[s] > x
-    while (lo < hi) {
-        const size_t mid = lo + (hi - lo) / 2;
-        if (*QSV_DBG(u + mid) > x) hi = mid; else lo = mid + 1;
-    }
-    return lo;
-}
-
+// Sixteen lanes a shot, shots in any order (a host sort of 100 000 shots and a second pass over the
+// whole register took 8 ms).  The chunk is the last whose offset lies below u; inside it the first group
+// of 16 threads, then the first of its threads, then the first amplitude whose running sum reaches u,
+// each running sum rounded as the chunk's scan rounds it.
 template <typename T>
-__global__ void __launch_bounds__(kChunkThreads) k_sample_chunks(const vec2_t<T>* __restrict__ s, uint64_t dim,
-                                                                 const double2* __restrict__ total_p,
-                                                                 const double* __restrict__ off, unsigned n_chunks,
-                                                                 const double* __restrict__ u, size_t n_shots,
-                                                                 uint64_t* __restrict__ out) {
-    __shared__ double sh[kChunkThreads];
-    __shared__ double cp[1 << kChunkLog];
-    __shared__ double tot;
-    const unsigned c = blockIdx.x;
-    // shots whose lower_bound lands in this chunk: off[c] < u <= off[c+1] (first/last chunk open)
-    const size_t lo = c == 0 ? 0 : first_greater(u, n_shots, *QSV_DBG(off + c));
-    const size_t hi = c + 1 == n_chunks ? n_shots : first_greater(u, n_shots, *QSV_DBG(off + (c + 1)));
-    if (lo >= hi) return;
-    double v[kPerThread];
-    const uint64_t start = static_cast<uint64_t>(c) << kChunkLog;
-    chunk_scan<T>(s, start, dim, 0.0, QSV_DBG(total_p)->x, v, sh, &tot);
-    const double off_c = *QSV_DBG(off + c);
-#pragma unroll
-    for (int r = 0; r < kPerThread; ++r) cp[threadIdx.x * kPerThread + r] = __dadd_rn(off_c, v[r]);
-    __syncthreads();
-    const uint64_t len = min(static_cast<uint64_t>(1) << kChunkLog, dim - start);
-    for (size_t sidx = lo + threadIdx.x; sidx < hi; sidx += blockDim.x) {
-        const double x = *QSV_DBG(u + sidx);
-        uint64_t a = 0, b = len;   // first j with cp[j] >= x
-        while (a < b) {
-            const uint64_t mid = (a + b) >> 1;
-            if (cp[mid] < x) a = mid + 1; else b = mid;
-        }
-        if (a >= len) a = len - 1;   // rounding past the chunk's last cumulative: stay in it
-        *QSV_DBG(out + sidx) = start + a;
+__global__ void __launch_bounds__(256) k_sample_shots(const vec2_t<T>* __restrict__ s, uint64_t dim,
+                                                      const double2* __restrict__ total_p, const double* __restrict__ off,
+                                                      unsigned n_chunks, const double* __restrict__ bases,
+                                                      const double* __restrict__ chunk_total, const double* __restrict__ u,
+                                                      size_t n_shots, uint64_t* __restrict__ out) {
+    static_assert(kPerThread == 16 && kGroups == 16, "half a warp holds a group");
+    const size_t shot = (static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 4;
+    const unsigned lane = threadIdx.x & 15u, upper = threadIdx.x & 16u;
+    const unsigned half = 0xffffu << upper;
+    if (shot >= n_shots) return;        // whole halves: every ballot and shuffle below names its half
+    const double x = *QSV_DBG(u + shot);
+    // c = how many of the offsets 1 .. n_chunks - 1 lie below x: 16 probes a round, not one
+    unsigned c = 0;
+    for (unsigned size = n_chunks - 1; size > 0;) {
+        const unsigned step = (size + 16) / 17, at = (lane + 1) * step - 1;
+        const unsigned below = __popc(__ballot_sync(half, at < size && x > *QSV_DBG(off + (c + min(at, size - 1) + 1))) & half);
+        c += below * step;
+        size = below == 16 ? size - 16 * step : min(step - 1, size - below * step);
     }
+    const double off_c = *QSV_DBG(off + c);
+    const uint64_t start = static_cast<uint64_t>(c) << kChunkLog;
+    const double* gb = bases + static_cast<uint64_t>(c) * kGroups;
+    const double end = *QSV_DBG(lane + 1 < kGroups ? gb + (lane + 1) : chunk_total + c);
+    const unsigned reach = (__ballot_sync(half, !(__dadd_rn(off_c, end) < x)) & half) >> upper;
+    const unsigned g = reach ? __ffs(reach) - 1 : kGroups - 1;
+    // the group's threads: this lane is thread 16 g + lane of the chunk's scan
+    const double total = QSV_DBG(total_p)->x;
+    __shared__ double turned[16][kGroups * (kPerThread + 1)];   // the block's 16 halves
+    double* q = turned[threadIdx.x >> 4];
+    const uint64_t group0 = start + static_cast<uint64_t>(g) * (kPerThread * kPerThread);
+#pragma unroll
+    for (int r = 0; r < kPerThread; ++r) {
+        const uint64_t i = group0 + r * kPerThread + lane;
+        q[r * (kPerThread + 1) + lane] = i < dim ? __ddiv_rn(prob<T>(*QSV_DBG(s + i)), total) : 0.0;
+    }
+    __syncwarp(half);
+    const uint64_t first = group0 + lane * kPerThread;
+    double v[kPerThread];
+    double run = 0;
+#pragma unroll
+    for (int r = 0; r < kPerThread; ++r) {
+        run = __dadd_rn(run, q[lane * (kPerThread + 1) + r]);
+        v[r] = run;
+    }
+    double acc = *QSV_DBG(gb + g), base = 0;
+#pragma unroll
+    for (int k = 0; k < kPerThread; ++k) {
+        if (lane == static_cast<unsigned>(k)) base = acc;
+        acc = __dadd_rn(acc, __shfl_sync(half, run, k, 16));
+    }
+    const unsigned here = (__ballot_sync(half, !(__dadd_rn(off_c, __dadd_rn(base, run)) < x)) & half) >> upper;
+    const unsigned owner = here ? __ffs(here) - 1 : kPerThread - 1;
+    if (lane != owner) return;
+    unsigned below = 0;
+#pragma unroll
+    for (int r = 0; r < kPerThread; ++r) below += __dadd_rn(off_c, __dadd_rn(base, v[r])) < x ? 1u : 0u;
+    // rounding past the chunk's last cumulative: stay in it
+    const uint64_t last = min(static_cast<uint64_t>(1) << kChunkLog, dim - start) - 1;
+    *QSV_DBG(out + shot) = min(first + below, start + last);
 }
 
 // ---------------------------------------------------------------- adjoint step
@@ -751,23 +835,26 @@ void scale_real(vec2_t<T>* s, int n, double f, cudaStream_t st) {
 }
 
 template <typename T>
-void sample_sorted(const vec2_t<T>* s, int n, const double* d_u, size_t n_shots, uint64_t* d_out,
-                   cudaStream_t st, Workspace& ws) {
+void sample_shots(const vec2_t<T>* s, int n, double* d_u, const uint32_t* seed, size_t n_shots, uint64_t* d_out,
+                  cudaStream_t st, Workspace& ws) {
     const uint64_t dim = 1ull << n;
     const unsigned n_chunks = static_cast<unsigned>((dim + (1ull << kChunkLog) - 1) >> kChunkLog);
-    const unsigned nb = red_blocks(dim);
-    // scratch layout: [partials nb+1 double2][chunk totals][offsets n_chunks+1]
-    const size_t bytes = (nb + 1) * sizeof(double2) + (2 * static_cast<size_t>(n_chunks) + 1) * sizeof(double);
+    const unsigned nb = red_blocks(dim), first = seed ? 1u : 0u;
+    // scratch layout: [partials nb+1 double2][chunk totals][offsets n_chunks+1][bases]
+    const size_t bytes = (nb + 1) * sizeof(double2) + ((2 + kGroups) * static_cast<size_t>(n_chunks) + 1) * sizeof(double);
     uint8_t* scr = static_cast<uint8_t*>(ws.scratch(bytes));
     double2* partials = reinterpret_cast<double2*>(scr);
     double* chunk_total = reinterpret_cast<double*>(scr + (nb + 1) * sizeof(double2));
     double* off = chunk_total + n_chunks;
+    double* bases = off + n_chunks + 1;
     k_prob_total<T><<<nb, kRed, 0, st>>>(s, dim, partials);
     k_final<<<1, kRed, 0, st>>>(partials, nb, partials + nb);
-    k_chunk_totals<T><<<n_chunks, kChunkThreads, 0, st>>>(s, dim, partials + nb, chunk_total);
+    k_chunk_totals<T><<<n_chunks + first, kChunkThreads, 0, st>>>(s, dim, partials + nb, chunk_total, bases, first,
+                                                                 seed ? *seed : 0u, d_u, n_shots);
     k_chunk_offsets<<<1, kOffThreads, 0, st>>>(chunk_total, n_chunks, off);
-    k_sample_chunks<T><<<n_chunks, kChunkThreads, 0, st>>>(s, dim, partials + nb, off, n_chunks, d_u,
-                                                          n_shots, d_out);
+    const size_t blocks = (n_shots + 15) / 16;
+    k_sample_shots<T><<<static_cast<unsigned>(blocks), 256, 0, st>>>(s, dim, partials + nb, off, n_chunks, bases, chunk_total,
+                                                                    d_u, n_shots, d_out);
     check_cuda(cudaGetLastError(), "sampling launch");
 }
 
@@ -817,8 +904,8 @@ template void inner<float, double>(const float2*, const double2*, int, cudaStrea
 template void inner<double, float>(const double2*, const float2*, int, cudaStream_t, Workspace&, double*);
 template void scale_real<double>(double2*, int, double, cudaStream_t);
 template void scale_real<float>(float2*, int, double, cudaStream_t);
-template void sample_sorted<double>(const double2*, int, const double*, size_t, uint64_t*, cudaStream_t, Workspace&);
-template void sample_sorted<float>(const float2*, int, const double*, size_t, uint64_t*, cudaStream_t, Workspace&);
+template void sample_shots<double>(const double2*, int, double*, const uint32_t*, size_t, uint64_t*, cudaStream_t, Workspace&);
+template void sample_shots<float>(const float2*, int, double*, const uint32_t*, size_t, uint64_t*, cudaStream_t, Workspace&);
 template void adjoint_param_step<double>(double2*, double2*, int, const AdjStep&, double*, unsigned, cudaStream_t);
 template void adjoint_param_step<float>(float2*, float2*, int, const AdjStep&, double*, unsigned, cudaStream_t);
 

@@ -254,10 +254,12 @@ void inner(const vec2_t<TA>* a, const vec2_t<TB>* b, int n, cudaStream_t st, Wor
 template <typename T>
 void scale_real(vec2_t<T>* s, int n, double f, cudaStream_t st);
 
-// terminal sampling: u sorted ascending (device), out_idx (device) in the same order
+// Terminal sampling, shots in any order: d_out[s] = the first index whose cumulative probability reaches
+// d_u[s].  With a seed the uniforms are drawn on the device into d_u (the reference's draws from
+// std::mt19937(seed), in shot order); without one d_u holds the caller's.
 template <typename T>
-void sample_sorted(const vec2_t<T>* s, int n, const double* d_u_sorted, size_t n_shots,
-                   uint64_t* d_out, cudaStream_t st, Workspace& ws);
+void sample_shots(const vec2_t<T>* s, int n, double* d_u, const uint32_t* seed, size_t n_shots, uint64_t* d_out,
+                  cudaStream_t st, Workspace& ws);
 
 // ---------------------------------------------------------------- readouts (kern_readout.cu)
 // Exact Born readout: counts the indices with |a|^2 > thr (returned); when d_keys is non-null

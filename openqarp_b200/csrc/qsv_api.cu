@@ -798,43 +798,44 @@ int qsv_uniforms(uint32_t seed, size_t n_shots, double* u) {
     });
 }
 
+// Shots from the register into `out`: the caller's uniforms, or (u null) the seed's draws.
+static void sample_to_host(Handle* h, const double* u, uint32_t seed, size_t n_shots, uint64_t* out) {
+    if (n_shots == 0) return;
+    if (!out) throw std::invalid_argument("null argument");
+    uint8_t* dev = static_cast<uint8_t*>(h->ws.shots(n_shots * 16));
+    double* d_u = reinterpret_cast<double*>(dev);
+    uint64_t* d_out = reinterpret_cast<uint64_t*>(dev + n_shots * 8);
+    if (u) check_cuda(cudaMemcpyAsync(d_u, u, n_shots * 8, cudaMemcpyHostToDevice, h->stream), "shots H2D");
+    const uint32_t* s = u ? nullptr : &seed;
+    if (h->dtype == QSV_C128) sample_shots<double>(S128(h), h->n, d_u, s, n_shots, d_out, h->stream, h->ws);
+    else sample_shots<float>(S64(h), h->n, d_u, s, n_shots, d_out, h->stream, h->ws);
+    constexpr size_t kStaged = size_t{1} << 20;     // up to 8 MiB through the kept pinned buffer
+    if (n_shots <= kStaged) {
+        double* stage = h->ws.host_result(n_shots);
+        check_cuda(cudaMemcpyAsync(stage, d_out, n_shots * 8, cudaMemcpyDeviceToHost, h->stream), "shots D2H");
+        check_cuda(cudaStreamSynchronize(h->stream), "sampling");
+        std::memcpy(out, stage, n_shots * 8);
+    } else {
+        d2h(h, out, d_out, n_shots * 8);
+    }
+    h->stats.launches += 5;
+}
+
 int qsv_sample(void* hp, const double* u, size_t n_shots, uint64_t* out) {
     return guarded([&] {
         Handle* h = H_(hp);
-        if (n_shots == 0) return;
-        if (!u || !out) throw std::invalid_argument("null argument");
-        std::vector<size_t> perm(n_shots);
-        std::iota(perm.begin(), perm.end(), size_t{0});
-        std::stable_sort(perm.begin(), perm.end(), [&](size_t a, size_t b) { return u[a] < u[b]; });
-        std::vector<double> us(n_shots);
-        for (size_t s = 0; s < n_shots; ++s) us[s] = u[perm[s]];
-        uint8_t* dev = static_cast<uint8_t*>(h->ws.shots(n_shots * 16));
-        double* d_u = reinterpret_cast<double*>(dev);
-        uint64_t* d_out = reinterpret_cast<uint64_t*>(dev + n_shots * 8);
-        check_cuda(cudaMemcpyAsync(d_u, us.data(), n_shots * 8, cudaMemcpyHostToDevice, h->stream), "shots H2D");
-        if (h->dtype == QSV_C128) sample_sorted<double>(S128(h), h->n, d_u, n_shots, d_out, h->stream, h->ws);
-        else sample_sorted<float>(S64(h), h->n, d_u, n_shots, d_out, h->stream, h->ws);
-        std::vector<uint64_t> idx(n_shots);
-        check_cuda(cudaMemcpyAsync(idx.data(), d_out, n_shots * 8, cudaMemcpyDeviceToHost, h->stream), "shots D2H");
-        check_cuda(cudaStreamSynchronize(h->stream), "sampling");
-        for (size_t s = 0; s < n_shots; ++s) out[perm[s]] = idx[s];
-        h->stats.launches += 5;
+        if (n_shots && !u) throw std::invalid_argument("null argument");
+        sample_to_host(h, u, 0, n_shots, out);
     });
 }
 
 int qsv_sample_seeded(void* hp, uint32_t seed, size_t n_shots, uint64_t* out) {
     Range range("qsv_sample_seeded");
-    std::vector<double> u(n_shots);
-    int rc = qsv_uniforms(seed, n_shots, u.data());
-    if (rc) return rc;
-    return qsv_sample(hp, u.data(), n_shots, out);
+    return guarded([&] { sample_to_host(H_(hp), nullptr, seed, n_shots, out); });
 }
 
 int qsv_sample_parities(void* hp, uint32_t seed, size_t n_shots, const uint64_t* zmasks, size_t n_masks,
                         uint64_t* odd) {
-    std::vector<double> u(n_shots);
-    int rc = qsv_uniforms(seed, n_shots, u.data());
-    if (rc) return rc;
     return guarded([&] {
         Handle* h = H_(hp);
         if (n_masks && (!zmasks || !odd)) throw std::invalid_argument("null argument");
@@ -842,8 +843,6 @@ int qsv_sample_parities(void* hp, uint32_t seed, size_t n_shots, const uint64_t*
             if (h->n < 64 && (zmasks[t] >> h->n) != 0)
                 throw std::invalid_argument("Z mask names a qubit outside the register");
         if (n_masks == 0) return;
-        // outcomes stay on the device in sorted-uniform order: parities do not depend on it
-        std::sort(u.begin(), u.end());
         uint8_t* dev = static_cast<uint8_t*>(h->ws.shots(n_shots * 16));
         double* d_u = reinterpret_cast<double*>(dev);
         uint64_t* d_out = reinterpret_cast<uint64_t*>(dev + n_shots * 8);
@@ -851,9 +850,8 @@ int qsv_sample_parities(void* hp, uint32_t seed, size_t n_shots, const uint64_t*
         auto* d_odd = reinterpret_cast<unsigned long long*>(d_masks + n_masks);
         check_cuda(cudaMemcpyAsync(d_masks, zmasks, n_masks * 8, cudaMemcpyHostToDevice, h->stream), "masks H2D");
         if (n_shots) {
-            check_cuda(cudaMemcpyAsync(d_u, u.data(), n_shots * 8, cudaMemcpyHostToDevice, h->stream), "shots H2D");
-            if (h->dtype == QSV_C128) sample_sorted<double>(S128(h), h->n, d_u, n_shots, d_out, h->stream, h->ws);
-            else sample_sorted<float>(S64(h), h->n, d_u, n_shots, d_out, h->stream, h->ws);
+            if (h->dtype == QSV_C128) sample_shots<double>(S128(h), h->n, d_u, &seed, n_shots, d_out, h->stream, h->ws);
+            else sample_shots<float>(S64(h), h->n, d_u, &seed, n_shots, d_out, h->stream, h->ws);
         }
         parity_counts(d_out, n_shots, d_masks, n_masks, d_odd, h->stream);
         check_cuda(cudaMemcpyAsync(odd, d_odd, n_masks * 8, cudaMemcpyDeviceToHost, h->stream), "parities D2H");
