@@ -225,11 +225,14 @@ struct Gen {
     bool has[kRtQubits] = {};
     // a factor owed by every amplitude of the tile: the bit-0 phases of normalised tables
     c128 cglob{1.0, 0.0};
-    // rotations of fixed gates (no parameter: their values do not change between parameter
-    // sets): `forms` hashes which of the two forms each takes; with `spec` the source carries
-    // only that form instead of a branch on the coefficient
-    bool spec = false;
-    uint64_t forms = 1469598103934665603ull;
+    // Bit-flip frame: the amplitude stored at local index i belongs to index i ^ (the bits with
+    // turned[b]).  A rotation by more than a quarter turn leaves its bit turned instead of moving
+    // data (gate_batch); every other op is rewritten for the stored index on the host, and the
+    // pass's store puts the amplitudes back (an XOR on the address).  Which bits are turned depends
+    // on the matrices, the source never does.
+    bool turned[kRtQubits] = {};
+    // deferred phases of qubits outside the tile (constants of the tile's base index)
+    std::vector<QubitPhase> outside;
     int normalised = 0;   // normalised tables since cglob was last applied
     double flops = 0;   // FP64 operations per thread per tile (FMA = 2, MUL = 1)
 
@@ -367,7 +370,7 @@ struct Gen {
     // in on qubits outside the tile (constants of the tile's base index), as one factor per
     // thread (starting from the tile constant), after the slot table; without lane, warp or
     // outside phases the slot table is the full one
-    void flush_all(const RtLayout& L, const std::vector<QubitPhase>& outside = {}) {
+    void flush_all(const RtLayout& L) {
         uint64_t m = 0, om = 0;
         for (int b = 0; b < kRtQubits; ++b) {
             if (!has[b]) continue;
@@ -415,20 +418,43 @@ struct Gen {
         o << "  }\n";
     }
 
+    // the deferred pair of qubit q (a tile bit's in the stored index), created as 1, 1
+    c128* owed(int q) {
+        const int b = local_of[q];
+        if (b >= 0) {
+            if (!has[b]) pend[b][0] = pend[b][1] = c128(1.0, 0.0);
+            has[b] = true;
+            return pend[b];
+        }
+        for (QubitPhase& x : outside)
+            if (x.q == q) return x.p;
+        QubitPhase x;
+        x.q = q;
+        x.p[0] = x.p[1] = c128(1.0, 0.0);
+        outside.push_back(x);
+        return outside.back().p;
+    }
+    bool turned_q(int q) const { return local_of[q] >= 0 && turned[local_of[q]]; }
+
     // consecutive one-qubit gates on distinct register slots: their D2 factors join the
     // deferred phases, one table applies them, then the real rotations; D1 is deferred.
     // A rotation is divided by its larger entry, so each output component is one FMA:
     //   c >= s:  R = c [[1, -t], [t, 1]],  t = s / c
-    //   s >  c:  R = s [[u, -1], [1, u]],  u = c / s
-    // the scale (c or s, the same for both basis states) joins the deferred phases, and the
-    // form is a uniform branch on a coefficient, so the kernel does not depend on the angles
+    //   s >  c:  R = s [[u, -1], [1, u]],  u = c / s, which is [[1, u], [-u, 1]] (the first form with
+    //            t = -u) whose outputs come exchanged, the second with its sign changed: the bit is
+    //            left turned and the sign joins D1
+    // the scale (c or s, the same for both basis states) joins the deferred phases.  One form serves
+    // every matrix, so a structure is compiled once and has no branch at a gate.  28-qubit brickwork
+    // with new matrices each call, whole call: 48.3 ms in complex128 and 33.1 ms in complex64;
+    // 52.8 and 38.0 ms with a uniform branch on the form at every gate.
     void gate_batch(const std::vector<const RtStep*>& gates, const RtLayout& L, int local_bit_of_slot[]) {
         std::vector<Factor1q> f;
         uint32_t smask = 0;
         for (const RtStep* st : gates) {
             const int p = st->slot_of[0];
             const int b = local_bit_of_slot[p];
-            f.push_back(factor_1q(st->op->m));
+            const std::vector<c128>& m = st->op->m;
+            f.push_back(factor_1q(turned[b] ? std::vector<c128>{m[3], m[2], m[1], m[0]} : m));
             const Factor1q& z = f.back();
             for (int v = 0; v < 2; ++v) pend[b][v] = (has[b] ? pend[b][v] : c128(1.0, 0.0)) * z.d2[v];
             has[b] = true;
@@ -441,59 +467,66 @@ struct Gen {
             const int b = local_bit_of_slot[p];
             const bool cos_form = f[i].c >= f[i].s;
             const double scale = cos_form ? f[i].c : f[i].s;
-            const double ratio = cos_form ? f[i].s / f[i].c : f[i].c / f[i].s;
-            const size_t at = push(c128(ratio, cos_form ? 0.0 : 1.0));
-            pend[b][0] = f[i].d1[0] * scale;
-            pend[b][1] = f[i].d1[1] * scale;
+            const size_t at = coef.size();
+            coef.push_back(cos_form ? f[i].s / f[i].c : -(f[i].c / f[i].s));
+            pend[b][0] = (cos_form ? f[i].d1[0] : f[i].d1[1]) * scale;
+            pend[b][1] = (cos_form ? f[i].d1[1] : -f[i].d1[0]) * scale;
             has[b] = true;
+            turned[b] ^= !cos_form;
             mark(0xB1u, static_cast<uint64_t>(p));
             flops += 8.0 * (kJitAmps / 2);
-            const bool fixed = gates[i]->op->fixed;
-            if (fixed) forms = (forms ^ (cos_form ? 0xC05u : 0x51Du)) * 1099511628211ull;
             if (!emit) continue;
-            // 0: branch on the coefficient, 1: cosine form only, 2: sine form only
-            const int only = (spec && fixed) ? (cos_form ? 1 : 2) : 0;
             const int B = 1 << p;
-            std::ostringstream a, bb;
-            if (f32) {
-                // complex64: each amplitude is one float2, and a rotation updates both of its
-                // components with one packed FMA (__ffma2_rn, rounding as fmaf per component)
-                for (int g = 0; g < kJitAmps; ++g) {
-                    if (g & B) continue;
-                    const std::string x0 = "a" + std::to_string(g), x1 = "a" + std::to_string(g | B);
-                    a << "    { const R2 y0 = " << x0 << "; " << x0 << " = __ffma2_rn(nt2, " << x1 << ", y0); "
-                      << x1 << " = __ffma2_rn(t2, y0, " << x1 << "); }\n";
-                    bb << "    { const R2 y0 = " << x0 << "; " << x0 << " = __ffma2_rn(t2, y0, make_float2(-" << x1
-                       << ".x, -" << x1 << ".y)); " << x1 << " = __ffma2_rn(t2, " << x1 << ", y0); }\n";
-                }
-                o << "  { const R t = " << cr(at) << "; const R2 t2 = make_float2(t, t), nt2 = make_float2(-t, -t);\n";
-                if (only == 1) o << a.str() << "  }\n";
-                else if (only == 2) o << bb.str() << "  }\n";
-                else o << "  if (" << ci(at) << " != 0) {\n" << bb.str() << "  } else {\n" << a.str() << "  } }\n";
-                continue;
-            }
+            o << "  { const R t = " << cr(at) << ";\n";
+            // complex64: each amplitude is one float2, and a rotation updates both of its
+            // components with one packed FMA (__ffma2_rn, rounding as fmaf per component)
+            if (f32) o << "    const R2 t2 = make_float2(t, t), nt2 = make_float2(-t, -t);\n";
             for (int g = 0; g < kJitAmps; ++g) {
                 if (g & B) continue;
                 const int h = g | B;
+                if (f32) {
+                    const std::string x0 = "a" + std::to_string(g), x1 = "a" + std::to_string(h);
+                    o << "    { const R2 y0 = " << x0 << "; " << x0 << " = __ffma2_rn(nt2, " << x1 << ", y0); "
+                      << x1 << " = __ffma2_rn(t2, y0, " << x1 << "); }\n";
+                    continue;
+                }
                 const std::string x0r = ar(g), x0i = ai(g), x1r = ar(h), x1i = ai(h);
-                a << "    { const R y0r = " << x0r << ", y0i = " << x0i << "; "
+                o << "    { const R y0r = " << x0r << ", y0i = " << x0i << "; "
                   << x0r << " = FMA(-t, " << x1r << ", y0r); " << x0i << " = FMA(-t, " << x1i << ", y0i); "
                   << x1r << " = FMA(t, y0r, " << x1r << "); " << x1i << " = FMA(t, y0i, " << x1i << "); }\n";
-                bb << "    { const R y0r = " << x0r << ", y0i = " << x0i << "; "
-                   << x0r << " = FMA(t, y0r, -" << x1r << "); " << x0i << " = FMA(t, y0i, -" << x1i << "); "
-                   << x1r << " = FMA(t, " << x1r << ", y0r); " << x1i << " = FMA(t, " << x1i << ", y0i); }\n";
             }
-            o << "  { const R t = " << cr(at) << ";\n";
-            if (only == 1) o << a.str() << "  }\n";
-            else if (only == 2) o << bb.str() << "  }\n";
-            else o << "  if (" << ci(at) << " != 0) {\n" << bb.str() << "  } else {\n" << a.str() << "  } }\n";
+            o << "  }\n";
         }
+    }
+
+    // Puts slot p's bit back where it is turned (a uniform branch on a coefficient): before ops whose
+    // form the host cannot rewrite.
+    void unturn_slot(const RtLayout& L, int p) {
+        const int b = L.reg[p];
+        const size_t at = coef.size();
+        coef.push_back(turned[b] ? 1.0 : 0.0);
+        if (turned[b]) std::swap(pend[b][0], pend[b][1]);
+        turned[b] = false;
+        mark(0xF7u, static_cast<uint64_t>(p));
+        if (!emit) return;
+        o << "  if (" << cr(at) << " != 0) {\n";
+        for (int g = 0; g < kJitAmps; ++g)
+            if (!(g & (1 << p))) swap_regs(g, g | (1 << p));
+        o << "  }\n";
+    }
+    void swap_regs(int g, int h) {
+        o << "    { const R xr = " << ar(g) << ", xi = " << ai(g) << "; " << ar(g) << " = " << ar(h) << "; " << ai(g) << " = "
+          << ai(h) << "; " << ar(h) << " = xr; " << ai(h) << " = xi; }\n";
     }
 
     void dense(const Op& op, const std::vector<int>& slot_of) {
         const int k = op.k, D = 1 << k;
         const size_t at = coef.size();
-        for (const c128& v : op.m) push(v);
+        int tm = 0;      // turned bits: rows and columns exchanged
+        for (int b = 0; b < k; ++b)
+            if (turned_q(static_cast<int>(op.qubits[b]))) tm |= 1 << b;
+        for (int y = 0; y < D; ++y)
+            for (int x = 0; x < D; ++x) push(op.m[static_cast<size_t>((y ^ tm) * D + (x ^ tm))]);
         uint32_t slots = 0;
         uint64_t so = 0;
         for (int b = 0; b < k; ++b) {
@@ -531,10 +564,34 @@ struct Gen {
         }
     }
 
+    // m0 on the amplitudes whose bits of op.mask are all 1.  One bit: deferred.  Two bits: with turned
+    // bits f and s = 1 - 2 f, (f1 + s1 b1)(f2 + s2 b2) is the phase of the stored bits, so the turned
+    // bits leave one-qubit phases and the pair's sign.  More: the turned bits are put back or flip
+    // their part of the condition.
     void phase(const Op& op, const RtLayout& L) {
+        const int width = __builtin_popcountll(op.mask);
+        c128 m0 = op.m[0];
+        const bool sign = m0 == c128(-1.0, 0.0);
+        if (width == 1) {
+            const int q = __builtin_ctzll(op.mask);
+            const bool t = turned_q(q);
+            owed(q)[t ? 0 : 1] *= m0;
+            mark(0xA3u, op.mask);
+            return;
+        }
+        if (width == 2) {
+            const int q1 = __builtin_ctzll(op.mask), q2 = 63 - __builtin_clzll(op.mask);
+            const bool f1 = turned_q(q1), f2 = turned_q(q2);
+            auto power = [&](int e) { return e == 0 ? c128(1.0, 0.0) : e > 0 ? m0 : 1.0 / m0; };
+            const int s1 = f1 ? -1 : 1, s2 = f2 ? -1 : 1;
+            // both pairs are touched whatever is turned: the structure does not depend on the matrices
+            owed(q1)[1] *= power(f2 ? s1 : 0);
+            owed(q2)[1] *= power(f1 ? s2 : 0);
+            if (f1 && f2) cglob *= m0;
+            m0 = sign ? m0 : power(s1 * s2);
+        }
         uint32_t rm = 0;
-        const std::string c = full_cond(L, op.mask, &rm);
-        const bool sign = op.m[0] == c128(-1.0, 0.0);
+        const std::string c = width == 2 ? full_cond(L, op.mask, &rm) : turned_cond(L, op.mask, &rm);
         mark(sign ? 0xA1u : 0xA2u, rm);
         if (sign && c.empty()) {
             if (emit)
@@ -552,7 +609,7 @@ struct Gen {
             o << "  }\n";
             return;
         }
-        const size_t at = push(op.m[0]);
+        const size_t at = push(m0);
         flops += 6.0 * static_cast<double>(kJitAmps >> __builtin_popcount(rm));
         if (!emit) return;
         o << "  if (" << (c.empty() ? "true" : c) << ") {\n";
@@ -561,11 +618,75 @@ struct Gen {
         o << "  }\n";
     }
 
-    void ctrl1(const Op& op, const RtLayout& L, uint8_t slots) {
+    // full_cond for ops that take the bits as they are: slot bits are put back, turned lane and warp
+    // bits compare with a coefficient
+    std::string turned_cond(const RtLayout& L, uint64_t gmask, uint32_t* rm) {
+        uint64_t out = 0;
+        const uint32_t lm = split(gmask, &out);
+        for (int b = 0; b < kRtQubits; ++b) {
+            int k = 0;
+            if (((lm >> b) & 1) && place(L, b, &k) == 'r') unturn_slot(L, k);
+        }
+        *rm = 0;
+        std::string c;
+        mark(lm, out);
+        if (out) c = "((base & " + hex64(out) + ") == " + hex64(out) + ")";
+        for (int b = 0; b < kRtQubits; ++b) {
+            if (!((lm >> b) & 1)) continue;
+            int k = 0;
+            const char w = place(L, b, &k);
+            if (w == 'r') {
+                *rm |= 1u << k;
+                continue;
+            }
+            const size_t at = coef.size();
+            coef.push_back(turned[b] ? 1.0 : 0.0);
+            c += (c.empty() ? "" : " && ") + std::string(w == 'l' ? "((((lane >> " : "((((warp >> ") + std::to_string(k) +
+                 ") & 1u) != 0u) != (" + cr(at) + " != 0))";
+        }
+        return c;
+    }
+
+    // A controlled X from one control moves data without arithmetic: a rename where the control is a
+    // slot bit, selects elsewhere.  A turned control applies X to the other half: the same exchange
+    // with the target left turned.
+    bool exchange(const Op& op, const RtLayout& L, uint8_t slots) {
+        const bool x = op.m[0] == c128(0.0, 0.0) && op.m[3] == c128(0.0, 0.0) && op.m[1] == c128(1.0, 0.0) &&
+                       op.m[2] == c128(1.0, 0.0);
+        if (!x || __builtin_popcountll(op.mask) != 1) return false;
         uint32_t rm = 0;
         const std::string c = full_cond(L, op.mask, &rm);
+        mark(0xC2u, slots);
+        if (turned_q(__builtin_ctzll(op.mask))) {
+            const int t = local_of[op.target];
+            turned[t] = !turned[t];
+            std::swap(pend[t][0], pend[t][1]);
+        }
+        if (!emit) return true;
+        const int tb = slots;
+        if (!c.empty()) o << "  { const bool on = " << c << ";\n";
+        for (int g = 0; g < kJitAmps; ++g) {
+            if ((g & tb) || (static_cast<uint32_t>(g) & rm) != rm) continue;
+            const int h = g | tb;
+            if (c.empty()) {
+                swap_regs(g, h);
+                continue;
+            }
+            o << "    { const R xr = " << ar(g) << ", xi = " << ai(g) << ", yr = " << ar(h) << ", yi = " << ai(h) << "; "
+              << ar(g) << " = on ? yr : xr; " << ai(g) << " = on ? yi : xi; " << ar(h) << " = on ? xr : yr; " << ai(h)
+              << " = on ? xi : yi; }\n";
+        }
+        if (!c.empty()) o << "  }\n";
+        return true;
+    }
+
+    void ctrl1(const Op& op, const RtLayout& L, uint8_t slots) {
+        if (exchange(op, L, slots)) return;
+        uint32_t rm = 0;
+        const std::string c = turned_cond(L, op.mask, &rm);
         const size_t at = coef.size();
-        for (int e = 0; e < 4; ++e) push(op.m[e]);
+        const bool t = turned_q(op.target);
+        for (int e = 0; e < 4; ++e) push(op.m[t ? 3 - e : e]);
         mark(0xC1u, slots);
         flops += 16.0 * (kJitAmps / 2);
         if (!emit) return;
@@ -584,8 +705,18 @@ struct Gen {
     }
 
     void diag(const Op& op, const RtLayout& L) {
+        uint32_t tm = 0;
+        for (int b = 0; b < op.k; ++b)
+            if (turned_q(static_cast<int>(op.qubits[b]))) tm |= 1u << b;
+        if (op.k == 1) {
+            const int q = static_cast<int>(op.qubits[0]);
+            c128* p = owed(q);
+            for (uint32_t v = 0; v < 2; ++v) p[v] *= op.m[v ^ tm];
+            mark(0xE1u, static_cast<uint64_t>(q));
+            return;
+        }
         const size_t at = coef.size();
-        for (const c128& v : op.m) push(v);
+        for (uint32_t v = 0; v < op.m.size(); ++v) push(op.m[v ^ tm]);
         // table index bit b <- qubit op.qubits[b]: slot bits are constants per register; lane,
         // warp and outside bits form a per-thread base index
         std::string thr = "0u";
@@ -643,7 +774,10 @@ struct Gen {
         }
         if (outz) tz += " ^ ((unsigned)__popcll(base & " + hex64(outz) + ") & 1u)";
         const int e = (__builtin_popcountll(op.mask & op.zmask) + 3) & 3;
-        const size_t at = push(op.m[0]);
+        bool odd = false;     // turned qubits under a Z or Y change the sign of s
+        for (int q = 0; q < 64; ++q)
+            if ((op.zmask >> q) & 1) odd ^= turned_q(q);
+        const size_t at = push(odd ? std::conj(op.m[0]) : op.m[0]);
         mark(0x9Au, xm | (zm << 8) | (static_cast<uint64_t>(e) << 16));
         mark(outz, static_cast<uint64_t>(lz));
         flops += 6.0 * kJitAmps;
@@ -760,16 +894,16 @@ constexpr bool kJitDebug = false;
 // coefficients.
 // A pass of a chain starts from the carry of the pass before (cin: phases on its tile qubits
 // become its own deferred phases, the others pass through) and, unless it ends the chain,
-// hands its deferred phases on (cout) instead of applying them.
+// hands its deferred phases on (cout) instead of applying them.  *turned: the qubits whose bits the
+// pass's store turns back.
 bool walk_pass(const TilePass& pass, const RtPlan& plan, int n, Gen* g, RtLayout* last, const Carry* cin,
-               bool final, Carry* cout) {
+               bool final, Carry* cout, uint64_t* turned) {
     if (!jit_capable(plan)) return false;
     for (int q = 0; q < 64; ++q) g->local_of[q] = -1;
     for (int j = 0; j < kRtQubits; ++j) g->local_of[pass.tile_qubits[j]] = j;
     g->mark(static_cast<uint64_t>(n), 0x715Eu);
     for (int j = 0; j < kRtQubits; ++j) g->mark(pass.tile_qubits[j]);
     g->mark_layout(plan.load);
-    std::vector<QubitPhase> through;   // carried phases of qubits outside the tile
     if (cin) {
         uint64_t in_mask = 0;
         for (const QubitPhase& x : cin->phases) {
@@ -779,7 +913,7 @@ bool walk_pass(const TilePass& pass, const RtPlan& plan, int n, Gen* g, RtLayout
                 g->pend[b][1] = x.p[1];
                 g->has[b] = true;
             } else {
-                through.push_back(x);
+                g->outside.push_back(x);
             }
             in_mask |= 1ull << x.q;
         }
@@ -805,6 +939,7 @@ bool walk_pass(const TilePass& pass, const RtPlan& plan, int n, Gen* g, RtLayout
                 std::swap(g->pend[a][0], g->pend[b][0]);
                 std::swap(g->pend[a][1], g->pend[b][1]);
                 std::swap(g->has[a], g->has[b]);
+                std::swap(g->turned[a], g->turned[b]);
                 g->mark(0x7Bu);
                 g->mark_layout(st.layout);
                 L = st.layout;
@@ -843,16 +978,20 @@ bool walk_pass(const TilePass& pass, const RtPlan& plan, int n, Gen* g, RtLayout
             default: return false;
         }
     }
+    *turned = 0;
+    for (int b = 0; b < kRtQubits; ++b)
+        if (g->turned[b]) *turned |= 1ull << pass.tile_qubits[b];
     if (final || !cout) {
-        g->flush_all(L, through);
+        g->flush_all(L);
     } else {
-        cout->phases = through;
+        cout->phases = g->outside;
         for (int b = 0; b < kRtQubits; ++b)
             if (g->has[b]) {
                 QubitPhase x;
                 x.q = static_cast<int>(pass.tile_qubits[b]);
-                x.p[0] = g->pend[b][0];
-                x.p[1] = g->pend[b][1];
+                // the store puts turned bits back
+                x.p[0] = g->pend[b][g->turned[b] ? 1 : 0];
+                x.p[1] = g->pend[b][g->turned[b] ? 0 : 1];
                 cout->phases.push_back(x);
             }
         std::sort(cout->phases.begin(), cout->phases.end(),
@@ -930,7 +1069,7 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
     }
     s << "struct __align__(8) C" << idx << " { R c[" << nc << "]; };\n"
       << "extern \"C\" __global__ void __launch_bounds__(" << kJitThreads << ", " << jit_ctas(f32)
-      << ") qsv_jit_" << idx << "(R2* __restrict__ s, u64 n_tiles, const __grid_constant__ C" << idx << " P"
+      << ") qsv_jit_" << idx << "(R2* __restrict__ s, u64 n_tiles, u64 turned, const __grid_constant__ C" << idx << " P"
       << (kJitDebug ? ", unsigned long long* __restrict__ dbg" : "") << ") {\n"
       << "  extern __shared__ __align__(16) unsigned char smem[];\n"
       << "  double2* xb = reinterpret_cast<double2*>(smem);\n"
@@ -968,11 +1107,12 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
       << "  if (t + gridDim.x < n_tiles) {\n    const u64 tn = t + gridDim.x;\n    const u64 b1 = " << deposit("tn")
       << ";\n" << issue("b1") << "  }\n"
       << "  asm volatile(\"cp.async.commit_group;\\n\" ::: \"memory\");\n";
+    s << "  const u64 to = (base | gfin) ^ turned;\n";
     for (int r = 0; r < kJitAmps; ++r) {
         uint64_t gc = 0;
         for (int p = 0; p < kRtRegBits; ++p)
             if ((r >> p) & 1) gc |= 1ull << tq[F.reg[p]];
-        s << "  __stcs(s + " << at("base | gfin | " + hex64(gc)) << ", MK(" << Gen::ar(r) << ", " << Gen::ai(r) << "));\n";
+        s << "  __stcs(s + " << at("to ^ " + hex64(gc)) << ", MK(" << Gen::ar(r) << ", " << Gen::ai(r) << "));\n";
     }
     s << "  }\n  asm volatile(\"cp.async.wait_group 0;\\n\" ::: \"memory\");\n}\n";
     return s.str();
@@ -980,16 +1120,14 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
 
 // Source (with emit) or only the signature and coefficients (without) of one pass.
 bool gen_pass(const TilePass& pass, const RtPlan& plan, int n, int idx, bool emit, bool f32, std::string* src,
-              std::vector<double>* coef, uint64_t* sig_hash, double* flops_per_amp = nullptr,
-              const Carry* cin = nullptr, bool final = true, Carry* cout = nullptr, bool spec = false,
-              uint64_t* forms = nullptr) {
+              std::vector<double>* coef, uint64_t* sig_hash, uint64_t* turned, double* flops_per_amp = nullptr,
+              const Carry* cin = nullptr, bool final = true, Carry* cout = nullptr) {
     Gen g;
     g.emit = emit;
     g.f32 = f32;
-    g.spec = spec;
     g.mark(f32 ? 0xF32u : 0xF64u);
     RtLayout last{};
-    if (!walk_pass(pass, plan, n, &g, &last, cin, final, cout)) return false;
+    if (!walk_pass(pass, plan, n, &g, &last, cin, final, cout, turned)) return false;
     uint64_t h = 1469598103934665603ull;
     for (uint64_t v : g.sig)
         for (int b = 0; b < 8; ++b) {
@@ -997,7 +1135,6 @@ bool gen_pass(const TilePass& pass, const RtPlan& plan, int n, int idx, bool emi
             h *= 1099511628211ull;
         }
     *sig_hash = h;
-    if (forms) *forms = g.forms;
     if (flops_per_amp) *flops_per_amp = g.flops / kJitAmps;
     if (emit) *src = pass_source(pass, plan, n, idx, g.o.str(), g.coef.size(), last, f32);
     coef->swap(g.coef);
@@ -1082,7 +1219,7 @@ struct PassWalk {
     bool has_cin = false;
     Carry cin;
     bool final = true;
-    uint64_t forms = 0;   // the fixed gates' rotation forms (Gen::forms)
+    uint64_t turned = 0;  // qubits the store turns back (walk_pass)
 };
 
 std::vector<PassWalk> walk_all(const std::vector<const TilePass*>& passes, std::vector<RtPlan>& plans, int n,
@@ -1095,8 +1232,7 @@ std::vector<PassWalk> walk_all(const std::vector<const TilePass*>& passes, std::
         if (!plan_rt(*passes[i], &plans[i], f32 ? 8 : 16)) continue;
         std::string unused;
         PassWalk& w = alone[i];
-        w.ok = gen_pass(*passes[i], plans[i], n, 0, false, f32, &unused, &w.coef, &w.sig, &w.flops_per_amp,
-                        nullptr, true, nullptr, false, &w.forms);
+        w.ok = gen_pass(*passes[i], plans[i], n, 0, false, f32, &unused, &w.coef, &w.sig, &w.turned, &w.flops_per_amp);
     }
     std::vector<PassWalk> chained(np);
     Carry cur;
@@ -1112,8 +1248,8 @@ std::vector<PassWalk> walk_all(const std::vector<const TilePass*>& passes, std::
         if (in_chain) w.cin = cur;
         Carry next;
         std::string unused;
-        w.ok = gen_pass(*passes[i], plans[i], n, 0, false, f32, &unused, &w.coef, &w.sig, &w.flops_per_amp,
-                        w.has_cin ? &w.cin : nullptr, w.final, w.final ? nullptr : &next, false, &w.forms);
+        w.ok = gen_pass(*passes[i], plans[i], n, 0, false, f32, &unused, &w.coef, &w.sig, &w.turned, &w.flops_per_amp,
+                        w.has_cin ? &w.cin : nullptr, w.final, w.final ? nullptr : &next);
         if (!w.ok) return alone;
         cur = std::move(next);
         in_chain = !w.final;
@@ -1122,27 +1258,6 @@ std::vector<PassWalk> walk_all(const std::vector<const TilePass*>& passes, std::
 }
 
 std::mutex g_jit_mu;
-
-// Compile-time rotation forms: a pass structure is compiled with its fixed gates' forms when it
-// is first seen; if the same structure later comes with other forms (fixed matrices that do
-// change between calls), it takes the branching kernel from then on, so a stream of new
-// matrices cannot force a compilation per call.  Guarded by g_jit_mu.
-std::map<uint64_t, uint64_t> g_first_forms;
-std::map<uint64_t, bool> g_unstable_forms;
-const uint64_t kNoForms = 1469598103934665603ull;
-
-bool specialise_forms(uint64_t sig, uint64_t forms) {
-    if (forms == kNoForms) return false;   // no fixed rotation in the pass
-    if (g_unstable_forms.count(sig)) return false;
-    auto it = g_first_forms.find(sig);
-    if (it == g_first_forms.end()) {
-        g_first_forms[sig] = forms;
-        return true;
-    }
-    if (it->second == forms) return true;
-    g_unstable_forms[sig] = true;
-    return false;
-}
 
 #ifdef QSV_DEBUG_BOUNDS
 // the compiled passes' fault words (count, first index), one per device, polled with the other
@@ -1213,6 +1328,7 @@ JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int devic
         PassWalk& w = walks[i];
         if (!w.ok) continue;
         out.flops_per_amp.push_back(w.flops_per_amp);
+        out.turned.push_back(w.turned);
         const uint64_t sig = w.sig ^ (static_cast<uint64_t>(major) << 56) ^ (static_cast<uint64_t>(minor) << 48);
         out.idx[i] = static_cast<int>(sigs.size());
         sigs.push_back(sig);
@@ -1230,15 +1346,6 @@ JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int devic
     }
     if (sigs.empty()) return out;
     std::lock_guard<std::mutex> lock(g_jit_mu);
-    // passes whose fixed rotations are compiled with their forms get their own kernel key
-    std::vector<char> spec(sigs.size(), 0);
-    for (size_t k = 0; k < sigs.size(); ++k) {
-        const uint64_t forms = walks[pass_of[k]].forms;
-        if (specialise_forms(sigs[k], forms)) {
-            spec[k] = 1;
-            sigs[k] ^= (forms * 0x9E3779B97F4A7C15ull) ^ 0x5BEC0000ull;
-        }
-    }
     std::vector<size_t> missing;
     for (size_t k = 0; k < sigs.size(); ++k)
         if (!g_kernels.count({sigs[k], ctx})) missing.push_back(k);
@@ -1253,10 +1360,10 @@ JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int devic
             const size_t i = pass_of[missing[j]];
             const PassWalk& w = walks[i];
             std::vector<double> coef;
-            uint64_t sig = 0;
+            uint64_t sig = 0, turned = 0;
             Carry next;
-            gen_pass(*passes[i], plans[i], n, 0, true, f32, &srcs[j], &coef, &sig, nullptr,
-                     w.has_cin ? &w.cin : nullptr, w.final, w.final ? nullptr : &next, spec[missing[j]] != 0);
+            gen_pass(*passes[i], plans[i], n, 0, true, f32, &srcs[j], &coef, &sig, &turned, nullptr,
+                     w.has_cin ? &w.cin : nullptr, w.final, w.final ? nullptr : &next);
             srcs[j] = std::string(kPrelude) + kPreludeDebug + srcs[j] + tag;
             char name[40];
             std::snprintf(name, sizeof name, "%016llx.cubin", static_cast<unsigned long long>(fnv1a(srcs[j])));
@@ -1309,11 +1416,12 @@ void jit_launch(const JitPlan& plan, int pass, void* s, int n, cudaStream_t st) 
     const unsigned grid = static_cast<unsigned>(
         std::min<unsigned long long>(n_tiles, static_cast<unsigned long long>(jit_ctas(plan.f32)) * sms));
     const std::vector<uint8_t>& c = plan.coef[static_cast<size_t>(k)];
+    unsigned long long turned = plan.turned[static_cast<size_t>(k)];
 #ifdef QSV_DEBUG_BOUNDS
     unsigned long long* dbg = jit_fault_word(device);
-    void* args[] = {&s, &n_tiles, const_cast<uint8_t*>(c.data()), &dbg};
+    void* args[] = {&s, &n_tiles, &turned, const_cast<uint8_t*>(c.data()), &dbg};
 #else
-    void* args[] = {&s, &n_tiles, const_cast<uint8_t*>(c.data())};
+    void* args[] = {&s, &n_tiles, &turned, const_cast<uint8_t*>(c.data())};
 #endif
     check_cu(driver().launch(static_cast<CUfunction>(plan.fns[static_cast<size_t>(k)]), grid, 1, 1, kJitThreads, 1, 1,
                              static_cast<unsigned>(jit_smem(plan.f32)),
@@ -1331,10 +1439,10 @@ std::string jit_source_for_test(const std::vector<const TilePass*>& passes, int 
         if (!w.ok) continue;
         std::string ps;
         std::vector<double> coef;
-        uint64_t sig = 0;
+        uint64_t sig = 0, turned = 0;
         Carry out;
-        if (!gen_pass(*passes[i], plans[i], n, next, true, f32, &ps, &coef, &sig, nullptr, w.has_cin ? &w.cin : nullptr,
-                      w.final, w.final ? nullptr : &out, w.forms != kNoForms))
+        if (!gen_pass(*passes[i], plans[i], n, next, true, f32, &ps, &coef, &sig, &turned, nullptr,
+                      w.has_cin ? &w.cin : nullptr, w.final, w.final ? nullptr : &out))
             continue;
         if (next > 0) {
             // one program holds every pass: the type definitions come once, with the first

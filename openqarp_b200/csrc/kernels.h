@@ -163,6 +163,7 @@ struct JitPlan {
     std::vector<int> idx;                   // per pass: kernel index, -1 = not compiled
     std::vector<std::vector<uint8_t>> coef; // per kernel: its coefficients (kernel parameters)
     std::vector<void*> fns;                 // per kernel: the loaded function (CUfunction)
+    std::vector<uint64_t> turned;           // per kernel: qubits whose bits the store flips (kernel parameter)
     std::vector<double> flops_per_amp;      // per kernel: FP64 operations per amplitude (FMA = 2)
 };
 JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int device, bool f32);

@@ -49,8 +49,7 @@ constexpr int kJitPlanSeeds = 32;
 // the circuit.  On a 28-qubit brickwork 12-qubit tiles then take 15 passes instead of the 25
 // that five mandatory low qubits leave.  Complex64 with four low qubits (128-byte runs) takes
 // 19 passes: its brickwork 24.5 against 23.9 ms, its 31-qubit Heisenberg chain 80.3 against
-// 79.4 ms a step (same box).  (Before the passes compiled fixed gates' rotation forms, the
-// chain ran 7 % faster with four.)
+// 79.4 ms a step (same box).
 inline int coalesced_low_qubits(int amp_bytes) {
     (void)amp_bytes;
     return 3;

@@ -1,0 +1,48 @@
+"""Compiled tile passes whose rotations turn by more than a quarter (their bits are left turned until
+the pass's store): every kind of op that then acts on turned bits - phases of one, two and more qubits,
+controlled gates of one and two controls, swaps, diagonals, Pauli rotations, dense blocks - on slot,
+lane, warp and outside qubits, in chains of passes, against the CPU oracle."""
+import numpy as np
+import pytest
+
+from openqarp_b200 import Command, GateType as G, Register, ir
+
+
+def _circuit(n, seed, count=260):
+    rng = np.random.default_rng([n, seed])
+    one = [G.X, G.Y, G.H, G.SX, G.Z, G.S, G.T]
+    rot = [G.Rx, G.Ry, G.Rz, G.P]
+    two = [G.CX, G.CX, G.CZ, G.CZ, G.CY, G.SWAP, G.CH, G.CSX]
+    tworot = [G.CP, G.CRx, G.CRz, G.RZZ, G.RXX, G.RYY]
+    out = []
+    for _ in range(count):
+        q = [int(x) for x in rng.permutation(n)[:4]]
+        pick = rng.integers(0, 12)
+        if pick < 2:
+            out.append(Command(one[rng.integers(len(one))], (q[0],)))
+        elif pick < 6:
+            out.append(Command(rot[rng.integers(len(rot))], (q[0],), (float(rng.uniform(-7, 7)),)))
+        elif pick < 8:
+            out.append(Command(two[rng.integers(len(two))], (q[0], q[1])))
+        elif pick < 10:
+            out.append(Command(tworot[rng.integers(len(tworot))], (q[0], q[1]), (float(rng.uniform(-7, 7)),)))
+        elif pick == 10:
+            out.append(Command([G.CCX, G.MCZ, G.CSWAP][rng.integers(3)], tuple(q[:3])))
+        else:
+            out.append(Command(G.U, (q[0],), tuple(float(x) for x in rng.uniform(-4, 4, 3))))
+    return out
+
+
+# a few hundred gates, each within 4 roundings of unit-norm amplitudes
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,tol", [("complex128", 1e-12), ("complex64", 2e-5)])
+@pytest.mark.parametrize("n,k", [(12, 0), (13, 1), (15, 0), (16, 2)])
+def test_turned_bits_match_oracle(restatement, n, k, dtype, tol):
+    for seed in (1, 2, 3):
+        buf = ir.pack(_circuit(n, seed)).buf
+        want = restatement.statevector(buf, n)
+        reg = Register(n, dtype)
+        reg.configure(k, 0, 3, 12)
+        reg.apply(buf)
+        assert np.max(np.abs(reg.get_state() - want)) < tol
+        reg.close()
