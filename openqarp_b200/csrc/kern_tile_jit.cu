@@ -138,6 +138,13 @@ constexpr int kJitCtasPerSm = 2;                          // complex128: 64 KiB 
 constexpr int kJitCtasPerSmF32 = 3;                       // complex64: 32 KiB, <= 85 registers
 int jit_ctas(bool f32) { return f32 ? kJitCtasPerSmF32 : kJitCtasPerSm; }
 size_t jit_smem(bool f32) { return (size_t{1} << kRtQubits) * (f32 ? 8 : 16); }
+// Pair passes (the adjoint's reverse sweep, complex128): psi and phi tiles and a column of accumulators
+// per thread; one CTA per SM, whose threads hold both tiles' 16 amplitudes (128 of 255 registers).  A
+// 24-qubit pass of some 21 inner products takes 0.35 ms, 3.1 TB/s: reading the tiles, the steps and the
+// stores of its one CTA follow one another.  The interpreter it replaces (1.6 ms) read and wrote both
+// tiles in shared memory at every step, with a barrier between.
+constexpr int kPairMaxAcc = 48;
+size_t pair_smem(int n_acc) { return 2 * jit_smem(false) + static_cast<size_t>(n_acc) * kJitThreads * sizeof(double); }
 
 uint32_t swz(uint32_t i) { return i ^ ((i >> 3 ^ i >> 6 ^ i >> 9) & 7u); }
 
@@ -243,8 +250,20 @@ struct Gen {
     }
     static std::string cr(size_t at) { return "P.c[" + std::to_string(at) + "]"; }
     static std::string ci(size_t at) { return "P.c[" + std::to_string(at + 1) + "]"; }
-    static std::string ar(int r) { return "a" + std::to_string(r) + "r"; }
-    static std::string ai(int r) { return "a" + std::to_string(r) + "i"; }
+    // `pair`: a pass of the adjoint's reverse sweep, every op on the registers of psi ("a") and of phi
+    // ("b"); the register names below are those of `set`
+    bool pair = false;
+    char set = 'a';
+    std::string ar(int r) const { return set + std::to_string(r) + "r"; }
+    std::string ai(int r) const { return set + std::to_string(r) + "i"; }
+    template <typename F>
+    void each_set(F&& f) {
+        f();
+        if (!pair) return;
+        set = 'b';
+        f();
+        set = 'a';
+    }
     void mark(uint64_t a, uint64_t b = 0) { sig.push_back(a); sig.push_back(b); }
     void mark_layout(const RtLayout& L) {
         uint64_t x = 0, y = 0;
@@ -357,13 +376,15 @@ struct Gen {
         }
         for (int j = 0; j < m; ++j) has[L.reg[slots[j]]] = false;
         if (!emit) return;
-        for (int r = 0; r < kJitAmps; ++r) {
-            int idx = 0;
-            for (int j = 0; j < m; ++j) idx |= ((r >> slots[j]) & 1) << j;
-            if (!full && idx == 0) continue;
-            const size_t e = at + 2 * static_cast<size_t>(full ? idx : idx - 1);
-            cmul_into(r, cr(e), ci(e));
-        }
+        each_set([&] {
+            for (int r = 0; r < kJitAmps; ++r) {
+                int idx = 0;
+                for (int j = 0; j < m; ++j) idx |= ((r >> slots[j]) & 1) << j;
+                if (!full && idx == 0) continue;
+                const size_t e = at + 2 * static_cast<size_t>(full ? idx : idx - 1);
+                cmul_into(r, cr(e), ci(e));
+            }
+        });
     }
 
     // end of a chain of passes: the deferred phases of lane and warp bits, and those carried
@@ -414,7 +435,9 @@ struct Gen {
               << ", pi = on ? " << ci(at + 2) << " : " << ci(at) << "; const R nr = fr * pr - fi * pi;"
               << " fi = fr * pi + fi * pr; fr = nr; }\n";
         }
-        for (int r = 0; r < kJitAmps; ++r) cmul_into(r, "fr", "fi");
+        each_set([&] {
+            for (int r = 0; r < kJitAmps; ++r) cmul_into(r, "fr", "fi");
+        });
         o << "  }\n";
     }
 
@@ -465,19 +488,31 @@ struct Gen {
         for (size_t i = 0; i < gates.size(); ++i) {
             const int p = gates[i]->slot_of[0];
             const int b = local_bit_of_slot[p];
-            const bool cos_form = f[i].c >= f[i].s;
-            const double scale = cos_form ? f[i].c : f[i].s;
-            const size_t at = coef.size();
-            coef.push_back(cos_form ? f[i].s / f[i].c : -(f[i].c / f[i].s));
-            pend[b][0] = (cos_form ? f[i].d1[0] : f[i].d1[1]) * scale;
-            pend[b][1] = (cos_form ? f[i].d1[1] : -f[i].d1[0]) * scale;
-            has[b] = true;
-            turned[b] ^= !cos_form;
-            mark(0xB1u, static_cast<uint64_t>(p));
-            flops += 8.0 * (kJitAmps / 2);
-            if (!emit) continue;
-            const int B = 1 << p;
-            o << "  { const R t = " << cr(at) << ";\n";
+            rotate(p, b, f[i].c, f[i].s, f[i].d1[0], f[i].d1[1]);
+        }
+    }
+
+    // diag(d0, d1) [[c, -s], [s, c]] on slot p holding local bit b, as above.  In a pair pass the scale
+    // joins the tile constant, so the deferred pairs stay unit phases and cancel in inner products.
+    void rotate(int p, int b, double c, double s, c128 d0, c128 d1) {
+        const bool cos_form = std::abs(c) >= std::abs(s);
+        double scale = cos_form ? c : s;
+        const size_t at = coef.size();
+        coef.push_back(cos_form ? s / c : -(c / s));
+        if (pair) {
+            cglob *= scale;
+            scale = 1.0;
+        }
+        pend[b][0] = (cos_form ? d0 : d1) * scale;
+        pend[b][1] = (cos_form ? d1 : -d0) * scale;
+        has[b] = true;
+        turned[b] ^= !cos_form;
+        mark(0xB1u, static_cast<uint64_t>(p));
+        flops += 8.0 * (kJitAmps / 2) * (pair ? 2 : 1);
+        if (!emit) return;
+        const int B = 1 << p;
+        o << "  { const R t = " << cr(at) << ";\n";
+        each_set([&] {
             // complex64: each amplitude is one float2, and a rotation updates both of its
             // components with one packed FMA (__ffma2_rn, rounding as fmaf per component)
             if (f32) o << "    const R2 t2 = make_float2(t, t), nt2 = make_float2(-t, -t);\n";
@@ -495,8 +530,8 @@ struct Gen {
                   << x0r << " = FMA(-t, " << x1r << ", y0r); " << x0i << " = FMA(-t, " << x1i << ", y0i); "
                   << x1r << " = FMA(t, y0r, " << x1r << "); " << x1i << " = FMA(t, y0i, " << x1i << "); }\n";
             }
-            o << "  }\n";
-        }
+        });
+        o << "  }\n";
     }
 
     // Puts slot p's bit back where it is turned (a uniform branch on a coefficient): before ops whose
@@ -510,8 +545,10 @@ struct Gen {
         mark(0xF7u, static_cast<uint64_t>(p));
         if (!emit) return;
         o << "  if (" << cr(at) << " != 0) {\n";
-        for (int g = 0; g < kJitAmps; ++g)
-            if (!(g & (1 << p))) swap_regs(g, g | (1 << p));
+        each_set([&] {
+            for (int g = 0; g < kJitAmps; ++g)
+                if (!(g & (1 << p))) swap_regs(g, g | (1 << p));
+        });
         o << "  }\n";
     }
     void swap_regs(int g, int h) {
@@ -536,6 +573,7 @@ struct Gen {
         mark(0xD0u + static_cast<uint64_t>(k), so);
         flops += static_cast<double>(kJitAmps / D) * D * D * 8.0;
         if (!emit) return;
+        each_set([&] {
         for (int g = 0; g < kJitAmps; ++g) {
             if (g & static_cast<int>(slots)) continue;
             std::vector<int> reg(D);
@@ -562,6 +600,7 @@ struct Gen {
             for (int y = 0; y < D; ++y) o << "    " << ar(reg[y]) << " = o" << y << "r; " << ai(reg[y]) << " = o" << y << "i;\n";
             o << "  }\n";
         }
+        });
     }
 
     // m0 on the amplitudes whose bits of op.mask are all 1.  One bit: deferred.  Two bits: with turned
@@ -594,18 +633,21 @@ struct Gen {
         const std::string c = width == 2 ? full_cond(L, op.mask, &rm) : turned_cond(L, op.mask, &rm);
         mark(sign ? 0xA1u : 0xA2u, rm);
         if (sign && c.empty()) {
-            if (emit)
+            if (emit) each_set([&] {
                 for (int r = 0; r < kJitAmps; ++r)
                     if ((static_cast<uint32_t>(r) & rm) == rm) o << "  " << ar(r) << " = -" << ar(r) << "; " << ai(r) << " = -" << ai(r) << ";\n";
+            });
             return;
         }
         if (sign) {
             // a sign flip under a runtime condition: XOR of the sign bits (integer pipe)
             if (!emit) return;
             o << "  { const int sm = (" << c << ") ? (int)0x80000000 : 0;\n";
-            for (int r = 0; r < kJitAmps; ++r)
-                if ((static_cast<uint32_t>(r) & rm) == rm)
-                    o << "    " << ar(r) << " = flip(" << ar(r) << ", sm); " << ai(r) << " = flip(" << ai(r) << ", sm);\n";
+            each_set([&] {
+                for (int r = 0; r < kJitAmps; ++r)
+                    if ((static_cast<uint32_t>(r) & rm) == rm)
+                        o << "    " << ar(r) << " = flip(" << ar(r) << ", sm); " << ai(r) << " = flip(" << ai(r) << ", sm);\n";
+            });
             o << "  }\n";
             return;
         }
@@ -613,8 +655,10 @@ struct Gen {
         flops += 6.0 * static_cast<double>(kJitAmps >> __builtin_popcount(rm));
         if (!emit) return;
         o << "  if (" << (c.empty() ? "true" : c) << ") {\n";
-        for (int r = 0; r < kJitAmps; ++r)
-            if ((static_cast<uint32_t>(r) & rm) == rm) cmul_into(r, cr(at), ci(at));
+        each_set([&] {
+            for (int r = 0; r < kJitAmps; ++r)
+                if ((static_cast<uint32_t>(r) & rm) == rm) cmul_into(r, cr(at), ci(at));
+        });
         o << "  }\n";
     }
 
@@ -665,17 +709,19 @@ struct Gen {
         if (!emit) return true;
         const int tb = slots;
         if (!c.empty()) o << "  { const bool on = " << c << ";\n";
-        for (int g = 0; g < kJitAmps; ++g) {
-            if ((g & tb) || (static_cast<uint32_t>(g) & rm) != rm) continue;
-            const int h = g | tb;
-            if (c.empty()) {
-                swap_regs(g, h);
-                continue;
+        each_set([&] {
+            for (int g = 0; g < kJitAmps; ++g) {
+                if ((g & tb) || (static_cast<uint32_t>(g) & rm) != rm) continue;
+                const int h = g | tb;
+                if (c.empty()) {
+                    swap_regs(g, h);
+                    continue;
+                }
+                o << "    { const R xr = " << ar(g) << ", xi = " << ai(g) << ", yr = " << ar(h) << ", yi = " << ai(h) << "; "
+                  << ar(g) << " = on ? yr : xr; " << ai(g) << " = on ? yi : xi; " << ar(h) << " = on ? xr : yr; " << ai(h)
+                  << " = on ? xi : yi; }\n";
             }
-            o << "    { const R xr = " << ar(g) << ", xi = " << ai(g) << ", yr = " << ar(h) << ", yi = " << ai(h) << "; "
-              << ar(g) << " = on ? yr : xr; " << ai(g) << " = on ? yi : xi; " << ar(h) << " = on ? xr : yr; " << ai(h)
-              << " = on ? xi : yi; }\n";
-        }
+        });
         if (!c.empty()) o << "  }\n";
         return true;
     }
@@ -692,6 +738,7 @@ struct Gen {
         if (!emit) return;
         const int tb = slots;
         o << "  if (" << (c.empty() ? "true" : c) << ") {\n";
+        each_set([&] {
         for (int g = 0; g < kJitAmps; ++g) {
             if ((g & tb) || (static_cast<uint32_t>(g) & rm) != rm) continue;
             const int h = g | tb;
@@ -701,6 +748,7 @@ struct Gen {
               << "      " << ar(h) << " = " << cr(at + 4) << " * x0r - " << ci(at + 4) << " * x0i + " << cr(at + 6) << " * x1r - " << ci(at + 6) << " * x1i;\n"
               << "      " << ai(h) << " = " << cr(at + 4) << " * x0i + " << ci(at + 4) << " * x0r + " << cr(at + 6) << " * x1i + " << ci(at + 6) << " * x1r; }\n";
         }
+        });
         o << "  }\n";
     }
 
@@ -740,6 +788,7 @@ struct Gen {
         flops += 6.0 * kJitAmps;
         if (!emit) return;
         o << "  { const unsigned di = " << thr << ";\n";
+        each_set([&] {
         for (int r = 0; r < kJitAmps; ++r) {
             uint32_t cst = 0;
             for (int b = 0; b < op.k; ++b)
@@ -748,6 +797,7 @@ struct Gen {
               << " const R xr = " << ar(r) << ", xi = " << ai(r) << "; "
               << ar(r) << " = pr * xr - pi * xi; " << ai(r) << " = pr * xi + pi * xr; }\n";
         }
+        });
         o << "  }\n";
     }
 
@@ -799,6 +849,7 @@ struct Gen {
         };
         o << "  { const unsigned tp = (" << tz << ") & 1u; const R c = " << cr(at) << ", sp = tp ? -" << ci(at)
           << " : " << ci(at) << ";\n";
+        each_set([&] {
         for (int g = 0; g < kJitAmps; ++g) {
             if (g & pivot) continue;
             const int h = g ^ static_cast<int>(xm);
@@ -810,6 +861,7 @@ struct Gen {
               << "      " << ar(g) << " = c * v" << g << "r + sp * " << hr << "; " << ai(g) << " = c * v" << g << "i + sp * " << hi << ";\n"
               << "      " << ar(h) << " = c * v" << h << "r + sp * " << gr << "; " << ai(h) << " = c * v" << h << "i + sp * " << gi << "; }\n";
         }
+        });
         o << "  }\n";
     }
 
@@ -818,7 +870,169 @@ struct Gen {
         mark(0x5Cu);
         flops += 6.0 * kJitAmps;
         if (!emit) return;
-        for (int r = 0; r < kJitAmps; ++r) cmul_into(r, cr(at), ci(at));
+        each_set([&] {
+            for (int r = 0; r < kJitAmps; ++r) cmul_into(r, cr(at), ci(at));
+        });
+    }
+
+    // ---- adjoint steps (pair passes).  A step's result is Im <phi|G|psi> (every generator's prefactor is
+    // imaginary), as a weighted sum of the pass's accumulators; with the deferred factors of the other
+    // qubits unit phases, the stored registers lack only |cglob|^2 of it.
+    struct AdjOut {
+        int slot;
+        std::vector<std::pair<int, double>> acc;   // (accumulator, weight)
+    };
+    std::vector<AdjOut> outs;
+    int n_acc = 0;
+
+    // Emits acc[a] += sum over (f, x, imag, sign) of sign * (Im or Re of conj(phi_f) psi_x), in four
+    // running sums so that neighbouring FMAs do not wait for one another.
+    struct Product {
+        int f, x;
+        bool imag, neg;
+    };
+    int accumulate(const std::vector<Product>& ps) {
+        const int a = n_acc++;
+        mark(0xAD1u, static_cast<uint64_t>(ps.size()));
+        for (const Product& q : ps) mark(static_cast<uint64_t>(q.f) | static_cast<uint64_t>(q.x) << 8, (q.imag ? 1u : 0u) | (q.neg ? 2u : 0u));
+        flops += 4.0 * static_cast<double>(ps.size());
+        if (!emit) return a;
+        o << "  { R v0 = 0, v1 = 0, v2 = 0, v3 = 0;\n";
+        for (size_t i = 0; i < ps.size(); ++i) {
+            const Product& q = ps[i];
+            const std::string fr = "b" + std::to_string(q.f) + "r", fi = "b" + std::to_string(q.f) + "i";
+            const std::string xr = "a" + std::to_string(q.x) + "r", xi = "a" + std::to_string(q.x) + "i";
+            const std::string v = "v" + std::to_string(i & 3);
+            const std::string p = q.neg ? "-" : "", m = q.neg ? "" : "-";
+            if (q.imag) o << "    " << v << " = FMA(" << p << fr << ", " << xi << ", " << v << "); " << v << " = FMA(" << m << fi << ", " << xr << ", " << v << ");\n";
+            else o << "    " << v << " = FMA(" << p << fr << ", " << xr << ", " << v << "); " << v << " = FMA(" << p << fi << ", " << xi << ", " << v << ");\n";
+        }
+        o << "    acc[" << a * kJitThreads << "u + tid] += (v0 + v1) + (v2 + v3); }\n";
+        return a;
+    }
+
+    enum AdjKind { ADJ_NONE, ADJ_DIAG, ADJ_X, ADJ_Y, ADJ_GENERAL };
+    static AdjKind adj_kind(const Op& op) {
+        if (op.k != 1) return ADJ_GENERAL;
+        const std::vector<c128>& G = op.g;
+        const bool off0 = G[1] == 0.0 && G[2] == 0.0;
+        if (off0 && G[0].imag() == 0 && G[3].imag() == 0 && op.m[1] == 0.0 && op.m[2] == 0.0) return ADJ_DIAG;
+        if (G[0] != 0.0 || G[3] != 0.0) return ADJ_NONE;
+        if (G[1] == G[2] && G[1].imag() == 0) return ADJ_X;
+        if (G[1] == -G[2] && G[1].real() == 0) return ADJ_Y;
+        return ADJ_NONE;
+    }
+    // diagonal generator and dagger: no data moves, the dagger is deferred
+    void adj_diag(const RtStep& st, const RtLayout& L) {
+        const Op& op = *st.op;
+        const int p = st.slot_of[0], b = L.reg[p], B = 1 << p;
+        const double w = std::norm(cglob);
+        const double z0 = op.g[turned[b] ? 3 : 0].real(), z1 = op.g[turned[b] ? 0 : 3].real();
+        AdjOut out{op.slot, {}};
+        std::vector<Product> half[2];
+        for (int r = 0; r < kJitAmps; ++r) half[(r & B) ? 1 : 0].push_back({r, r, true, false});
+        mark(0xAD2u, static_cast<uint64_t>(p));
+        if (op.g[0] == -op.g[3]) {
+            for (Product& q : half[1]) q.neg = true;
+            half[0].insert(half[0].end(), half[1].begin(), half[1].end());
+            out.acc.push_back({accumulate(half[0]), w * z0});
+        } else {
+            out.acc.push_back({accumulate(half[0]), w * z0});
+            out.acc.push_back({accumulate(half[1]), w * z1});
+        }
+        outs.push_back(std::move(out));
+        c128* o2 = owed(static_cast<int>(op.qubits[0]));
+        o2[0] *= op.m[turned[b] ? 3 : 0];
+        o2[1] *= op.m[turned[b] ? 0 : 3];
+    }
+    // off-diagonal generator: the inner product only (slot phases flushed); the dagger follows
+    void adj_off(const RtStep& st, const RtLayout& L, AdjKind kind) {
+        const Op& op = *st.op;
+        const int p = st.slot_of[0], b = L.reg[p], B = 1 << p;
+        // X: Im conj(phi0) psi1 + Im conj(phi1) psi0 times g; Y: Re conj(phi1) psi0 - Re conj(phi0) psi1
+        // times Im g10.  On a turned bit Y changes sign.
+        double w = std::norm(cglob) * (kind == ADJ_X ? op.g[2].real() : op.g[2].imag());
+        if (kind == ADJ_Y && turned[b]) w = -w;
+        std::vector<Product> ps;
+        for (int g = 0; g < kJitAmps; ++g) {
+            if (g & B) continue;
+            ps.push_back({g, g | B, kind == ADJ_X, kind == ADJ_Y});
+            ps.push_back({g | B, g, kind == ADJ_X, false});
+        }
+        mark(0xAD3u, static_cast<uint64_t>(p) | static_cast<uint64_t>(kind) << 8);
+        outs.push_back({op.slot, {{accumulate(ps), w}}});
+    }
+    // two-qubit (or global phase) generator with entries 0, +-1, +-i, then its dagger
+    bool adj_general(const RtStep& st, const RtLayout& L) {
+        const Op& op = *st.op;
+        flush_slots(L);
+        for (int b = 0; b < op.k; ++b) unturn_slot(L, st.slot_of[b]);
+        uint32_t slots = 0;
+        for (int b = 0; b < op.k; ++b) slots |= 1u << st.slot_of[b];
+        const int D = 1 << op.k;
+        std::vector<Product> ps;
+        for (int g = 0; g < kJitAmps; ++g) {
+            if (g & static_cast<int>(slots)) continue;
+            auto reg = [&](int x) {
+                int r = g;
+                for (int b = 0; b < op.k; ++b)
+                    if ((x >> b) & 1) r |= 1 << st.slot_of[b];
+                return r;
+            };
+            for (int y = 0; y < D; ++y)
+                for (int x = 0; x < D; ++x) {
+                    const c128 e = op.g[static_cast<size_t>(y * D + x)];
+                    if (e == 0.0) continue;
+                    if (std::abs(e.real()) == 1.0 && e.imag() == 0) ps.push_back({reg(y), reg(x), true, e.real() < 0});
+                    else if (std::abs(e.imag()) == 1.0 && e.real() == 0) ps.push_back({reg(y), reg(x), false, e.imag() < 0});
+                    else return false;
+                }
+        }
+        mark(0xAD4u, slots);
+        const double w = std::norm(cglob);
+        outs.push_back({op.slot, {{accumulate(ps), w}}});
+        if (op.k == 0) cglob *= op.m[0];
+        else dense(op, st.slot_of);
+        return true;
+    }
+    // One-qubit steps between layout changes act on distinct slots or in order on one: per round, every
+    // slot's leading diagonal steps (no data moves), then one rotation per slot behind one phase table.
+    bool one_qubit_run(const std::vector<const RtStep*>& run, const RtLayout& L) {
+        std::vector<const RtStep*> queue[kRtRegBits];
+        for (const RtStep* st : run) queue[st->slot_of[0]].push_back(st);
+        size_t at[kRtRegBits] = {};
+        for (;;) {
+            std::vector<const RtStep*> heads;
+            for (int p = 0; p < kRtRegBits; ++p) {
+                while (at[p] < queue[p].size() && queue[p][at[p]]->kind == RT_ADJ && adj_kind(*queue[p][at[p]]->op) == ADJ_DIAG)
+                    adj_diag(*queue[p][at[p]++], L);
+                if (at[p] < queue[p].size()) heads.push_back(queue[p][at[p]++]);
+            }
+            if (heads.empty()) return true;
+            flush_slots(L);
+            std::vector<const RtStep*> complex_gates;
+            int bit_of_slot[kRtRegBits];
+            for (int p = 0; p < kRtRegBits; ++p) bit_of_slot[p] = L.reg[p];
+            for (const RtStep* st : heads) {
+                const std::vector<c128>& m = st->op->m;
+                if (st->kind == RT_ADJ) {
+                    const AdjKind kind = adj_kind(*st->op);
+                    if (kind != ADJ_X && kind != ADJ_Y) return false;
+                    adj_off(*st, L, kind);
+                }
+                const bool real_rotation = m[0].imag() == 0 && m[1].imag() == 0 && m[2].imag() == 0 && m[3].imag() == 0 &&
+                                           m[0] == m[3] && m[1] == -m[2];
+                mark(0xAD5u, real_rotation ? 1u : 0u);
+                if (!real_rotation) {
+                    complex_gates.push_back(st);
+                    continue;
+                }
+                // [[c, -s], [s, c]] needs no phases before it (on a turned bit s changes sign)
+                const int p = st->slot_of[0], b = L.reg[p];
+                rotate(p, b, m[0].real(), turned[b] ? -m[2].real() : m[2].real(), 1.0, 1.0);
+            }
+            if (!complex_gates.empty()) gate_batch(complex_gates, L, bit_of_slot);
+        }
     }
 
     // shared-memory slot of register r in layout L: complex128 amplitudes take one 16-byte slot
@@ -828,9 +1042,9 @@ struct Gen {
         if (!f32) return "const unsigned sf = swz(" + lfix_expr(L) + ");";
         return "const unsigned lf = " + lfix_expr(L) + "; const unsigned sf = swz(lf >> 1), e0 = lf & 1u;";
     }
-    static std::string slot_of(const RtLayout& L, int r, bool f32) {
+    static std::string slot_of(const RtLayout& L, int r, bool f32, char set = 'a') {
         const uint32_t lr = reg_local(L, r);
-        if (!f32) return "xb[sf ^ " + std::to_string(swz(lr)) + "u]";
+        if (!f32) return std::string(set == 'a' ? "xb" : "yb") + "[sf ^ " + std::to_string(swz(lr)) + "u]";
         return "xf[2u * (sf ^ " + std::to_string(swz(lr >> 1)) + "u) + (e0 ^ " + std::to_string(lr & 1u) + "u)]";
     }
 
@@ -842,11 +1056,15 @@ struct Gen {
         if (!emit) return;
         if (!first) o << "  __syncthreads();\n";
         o << "  { " << slot_setup(from, f32) << "\n";
-        for (int r = 0; r < kJitAmps; ++r)
-            o << "    " << slot_of(from, r, f32) << " = MK(" << ar(r) << ", " << ai(r) << ");\n";
+        each_set([&] {
+            for (int r = 0; r < kJitAmps; ++r)
+                o << "    " << slot_of(from, r, f32, set) << " = MK(" << ar(r) << ", " << ai(r) << ");\n";
+        });
         o << "  }\n  __syncthreads();\n  { " << slot_setup(to, f32) << "\n";
-        for (int r = 0; r < kJitAmps; ++r)
-            o << "    { const R2 x = " << slot_of(to, r, f32) << "; " << ar(r) << " = x.x; " << ai(r) << " = x.y; }\n";
+        each_set([&] {
+            for (int r = 0; r < kJitAmps; ++r)
+                o << "    { const R2 x = " << slot_of(to, r, f32, set) << "; " << ar(r) << " = x.x; " << ai(r) << " = x.y; }\n";
+        });
         o << "  }\n";
     }
 };
@@ -855,7 +1073,7 @@ struct Gen {
 bool jit_capable(const RtPlan& plan) {
     for (const RtStep& s : plan.steps)
         if (s.kind != RT_XPOSE && s.kind != RT_RELABEL && s.kind != RT_DENSE && s.kind != RT_PHASE &&
-            s.kind != RT_CTRL1 && s.kind != RT_DIAG && s.kind != RT_SCALE && s.kind != RT_PAULI)
+            s.kind != RT_CTRL1 && s.kind != RT_DIAG && s.kind != RT_SCALE && s.kind != RT_PAULI && s.kind != RT_ADJ)
             return false;
     return true;
 }
@@ -945,8 +1163,18 @@ bool walk_pass(const TilePass& pass, const RtPlan& plan, int n, Gen* g, RtLayout
                 L = st.layout;
                 break;
             }
+            case RT_ADJ:
             case RT_DENSE:
-                if (st.op->k == 1) {
+                if (g->pair && st.op->k == 1) {
+                    std::vector<const RtStep*> run;
+                    size_t j = i;
+                    for (; j < ns && (plan.steps[j].kind == RT_DENSE || plan.steps[j].kind == RT_ADJ) && plan.steps[j].op->k == 1; ++j)
+                        run.push_back(&plan.steps[j]);
+                    if (!g->one_qubit_run(run, L)) return false;
+                    i = j - 1;
+                } else if (st.kind == RT_ADJ) {
+                    if (!g->adj_general(st, L)) return false;
+                } else if (st.op->k == 1) {
                     std::vector<const RtStep*> batch;
                     uint32_t used = 0;
                     size_t j = i;
@@ -1010,7 +1238,10 @@ bool walk_pass(const TilePass& pass, const RtPlan& plan, int n, Gen* g, RtLayout
 // amplitudes per thread, 32 KiB, three CTAs per SM (85 registers; 31.6 ms against 34.4 ms with
 // two on the 28-qubit brickwork, and four no faster).
 std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx, const std::string& steps,
-                        size_t n_coef, const RtLayout& F, bool f32) {
+                        size_t n_coef, const RtLayout& F, bool f32, bool pair, int n_acc) {
+    const std::string sets = pair ? "ab" : "a";
+    auto re = [](char set, int r) { return set + std::to_string(r) + "r"; };
+    auto im = [](char set, int r) { return set + std::to_string(r) + "i"; };
     const size_t nc = std::max<size_t>(n_coef, 1);
     // tile base: the bits of t deposited into the non-tile qubit positions, ascending
     std::vector<int> outside;
@@ -1055,8 +1286,9 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
             uint64_t gj = 0;
             for (int b2 = 0; b2 < 4 && 8 + low + b2 < kRtQubits; ++b2)
                 if ((j >> b2) & 1) gj |= 1ull << tq[8 + low + b2];
-            x << "    cp16(xb + (stid ^ " << swz(static_cast<uint32_t>(j) * kJitThreads) << "u), s + "
-              << at("(" + b + ") | gtid | " + hex64(gj)) << ");\n";
+            for (char set : sets)
+                x << "    cp16(" << (set == 'a' ? "xb" : "yb") << " + (stid ^ " << swz(static_cast<uint32_t>(j) * kJitThreads)
+                  << "u), " << (set == 'a' ? "s" : "s2") << " + " << at("(" + b + ") | gtid | " + hex64(gj)) << ");\n";
         }
         return x.str();
     };
@@ -1068,13 +1300,18 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
         s << "typedef double R; typedef double2 R2;\n#define FMA fma\n#define MK make_double2\n";
     }
     s << "struct __align__(8) C" << idx << " { R c[" << nc << "]; };\n"
-      << "extern \"C\" __global__ void __launch_bounds__(" << kJitThreads << ", " << jit_ctas(f32)
-      << ") qsv_jit_" << idx << "(R2* __restrict__ s, u64 n_tiles, u64 turned, const __grid_constant__ C" << idx << " P"
+      << "extern \"C\" __global__ void __launch_bounds__(" << kJitThreads << ", " << (pair ? 1 : jit_ctas(f32))
+      << ") qsv_jit_" << idx << "(R2* __restrict__ s, u64 n_tiles, u64 turned, "
+      << (pair ? "R2* __restrict__ s2, double2* __restrict__ partials, " : "") << "const __grid_constant__ C" << idx << " P"
       << (kJitDebug ? ", unsigned long long* __restrict__ dbg" : "") << ") {\n"
       << "  extern __shared__ __align__(16) unsigned char smem[];\n"
       << "  double2* xb = reinterpret_cast<double2*>(smem);\n"
-      << "  R2* xf = reinterpret_cast<R2*>(smem);\n"
-      << "  const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;\n"
+      << "  R2* xf = reinterpret_cast<R2*>(smem);\n";
+    if (pair)
+        s << "  double2* yb = xb + " << (1 << kRtQubits) << ";\n  double* acc = reinterpret_cast<double*>(yb + "
+          << (1 << kRtQubits) << ");\n  for (unsigned k = 0; k < " << n_acc << "u; ++k) acc[k * " << kJitThreads
+          << "u + threadIdx.x] = 0;\n";
+    s << "  const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;\n"
       << "  const u64 gtid = " << gtid << ";\n"
       << "  const unsigned stid = swz(tid);\n"
       << "  const u64 gfin = " << gfin << ";\n"
@@ -1092,12 +1329,14 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
         for (int r = 0; r < kJitAmps; ++r) s << (r ? ", a" : "a") << r;
     } else {
         s << "R ";
-        for (int r = 0; r < kJitAmps; ++r) s << (r ? ", " : "") << Gen::ar(r) << ", " << Gen::ai(r);
+        for (char set : sets)
+            for (int r = 0; r < kJitAmps; ++r) s << (r || set == 'b' ? ", " : "") << re(set, r) << ", " << im(set, r);
     }
     s << ";\n  { " << Gen::slot_setup(plan.load, f32) << "\n";
-    for (int r = 0; r < kJitAmps; ++r)
-        s << "    { const R2 x = " << Gen::slot_of(plan.load, r, f32) << "; " << Gen::ar(r) << " = x.x; "
-          << Gen::ai(r) << " = x.y; }\n";
+    for (char set : sets)
+        for (int r = 0; r < kJitAmps; ++r)
+            s << "    { const R2 x = " << Gen::slot_of(plan.load, r, f32, set) << "; " << re(set, r) << " = x.x; "
+              << im(set, r) << " = x.y; }\n";
     // one buffer serves the tile's loads and its transposes: the next tile's copies start once
     // the last transpose has been read, and run under this tile's stores (and the other CTAs
     // on the SM compute meanwhile)
@@ -1112,22 +1351,34 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
         uint64_t gc = 0;
         for (int p = 0; p < kRtRegBits; ++p)
             if ((r >> p) & 1) gc |= 1ull << tq[F.reg[p]];
-        s << "  __stcs(s + " << at("to ^ " + hex64(gc)) << ", MK(" << Gen::ar(r) << ", " << Gen::ai(r) << "));\n";
+        for (char set : sets)
+            s << "  __stcs(" << (set == 'a' ? "s" : "s2") << " + " << at("to ^ " + hex64(gc)) << ", MK(" << re(set, r) << ", "
+              << im(set, r) << "));\n";
     }
-    s << "  }\n  asm volatile(\"cp.async.wait_group 0;\\n\" ::: \"memory\");\n}\n";
+    s << "  }\n  asm volatile(\"cp.async.wait_group 0;\\n\" ::: \"memory\");\n";
+    if (pair)
+        s << "  __syncthreads();\n  for (unsigned k = warp; k < " << n_acc << "u; k += " << kJitThreads / 32 << "u) {\n"
+          << "    double v = 0;\n    for (unsigned j = lane; j < " << kJitThreads << "u; j += 32u) v += acc[k * " << kJitThreads
+          << "u + j];\n    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);\n"
+          << "    if (lane == 0) partials[(u64)k * gridDim.x + blockIdx.x] = make_double2(v, 0);\n  }\n";
+    s << "}\n";
     return s.str();
 }
 
-// Source (with emit) or only the signature and coefficients (without) of one pass.
-bool gen_pass(const TilePass& pass, const RtPlan& plan, int n, int idx, bool emit, bool f32, std::string* src,
+// Source (with emit) or only the signature and coefficients (without) of one pass; `pair`: a pass of the
+// reverse sweep, with its adjoint steps' results in `outs`.
+bool gen_pass(const TilePass& pass, const RtPlan& plan, int n, int idx, bool emit, bool f32, bool pair, std::string* src,
               std::vector<double>* coef, uint64_t* sig_hash, uint64_t* turned, double* flops_per_amp = nullptr,
-              const Carry* cin = nullptr, bool final = true, Carry* cout = nullptr) {
+              const Carry* cin = nullptr, bool final = true, Carry* cout = nullptr, std::vector<Gen::AdjOut>* outs = nullptr,
+              int* n_acc = nullptr) {
     Gen g;
     g.emit = emit;
     g.f32 = f32;
-    g.mark(f32 ? 0xF32u : 0xF64u);
+    g.pair = pair;
+    g.mark(pair ? 0xFADu : f32 ? 0xF32u : 0xF64u);
     RtLayout last{};
     if (!walk_pass(pass, plan, n, &g, &last, cin, final, cout, turned)) return false;
+    if (g.n_acc > kPairMaxAcc) return false;
     uint64_t h = 1469598103934665603ull;
     for (uint64_t v : g.sig)
         for (int b = 0; b < 8; ++b) {
@@ -1136,7 +1387,9 @@ bool gen_pass(const TilePass& pass, const RtPlan& plan, int n, int idx, bool emi
         }
     *sig_hash = h;
     if (flops_per_amp) *flops_per_amp = g.flops / kJitAmps;
-    if (emit) *src = pass_source(pass, plan, n, idx, g.o.str(), g.coef.size(), last, f32);
+    if (emit) *src = pass_source(pass, plan, n, idx, g.o.str(), g.coef.size(), last, f32, pair, g.n_acc);
+    if (outs) outs->swap(g.outs);
+    if (n_acc) *n_acc = g.n_acc;
     coef->swap(g.coef);
     if (coef->empty()) coef->push_back(0.0);
     return true;
@@ -1220,10 +1473,12 @@ struct PassWalk {
     Carry cin;
     bool final = true;
     uint64_t turned = 0;  // qubits the store turns back (walk_pass)
+    std::vector<Gen::AdjOut> outs;
+    int n_acc = 0;
 };
 
 std::vector<PassWalk> walk_all(const std::vector<const TilePass*>& passes, std::vector<RtPlan>& plans, int n,
-                               bool f32) {
+                               bool f32, bool pair = false) {
     const size_t np = passes.size();
     plans.assign(np, RtPlan{});
     std::vector<PassWalk> alone(np);
@@ -1232,7 +1487,8 @@ std::vector<PassWalk> walk_all(const std::vector<const TilePass*>& passes, std::
         if (!plan_rt(*passes[i], &plans[i], f32 ? 8 : 16)) continue;
         std::string unused;
         PassWalk& w = alone[i];
-        w.ok = gen_pass(*passes[i], plans[i], n, 0, false, f32, &unused, &w.coef, &w.sig, &w.turned, &w.flops_per_amp);
+        w.ok = gen_pass(*passes[i], plans[i], n, 0, false, f32, pair, &unused, &w.coef, &w.sig, &w.turned,
+                        &w.flops_per_amp, nullptr, true, nullptr, &w.outs, &w.n_acc);
     }
     std::vector<PassWalk> chained(np);
     Carry cur;
@@ -1248,8 +1504,8 @@ std::vector<PassWalk> walk_all(const std::vector<const TilePass*>& passes, std::
         if (in_chain) w.cin = cur;
         Carry next;
         std::string unused;
-        w.ok = gen_pass(*passes[i], plans[i], n, 0, false, f32, &unused, &w.coef, &w.sig, &w.turned, &w.flops_per_amp,
-                        w.has_cin ? &w.cin : nullptr, w.final, w.final ? nullptr : &next);
+        w.ok = gen_pass(*passes[i], plans[i], n, 0, false, f32, pair, &unused, &w.coef, &w.sig, &w.turned,
+                        &w.flops_per_amp, w.has_cin ? &w.cin : nullptr, w.final, w.final ? nullptr : &next, &w.outs, &w.n_acc);
         if (!w.ok) return alone;
         cur = std::move(next);
         in_chain = !w.final;
@@ -1308,9 +1564,10 @@ std::map<std::pair<uint64_t, CUcontext>, CUfunction> g_kernels;
 
 // ---------------------------------------------------------------- public
 
-JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int device, bool f32) {
+JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int device, bool f32, bool pair) {
     JitPlan out;
     out.f32 = f32;
+    out.pair = pair;
     out.idx.assign(passes.size(), -1);
     int major = 0, minor = 0;
     check_cuda(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device), "compute capability");
@@ -1323,12 +1580,20 @@ JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int devic
     std::vector<size_t> pass_of;
     std::vector<uint64_t> sigs;
     std::vector<RtPlan> plans;
-    std::vector<PassWalk> walks = walk_all(passes, plans, n, f32);
+    std::vector<PassWalk> walks = walk_all(passes, plans, n, f32, pair);
     for (size_t i = 0; i < passes.size(); ++i) {
         PassWalk& w = walks[i];
+        if (!w.ok && pair && !passes[i]->tile_qubits.empty()) return JitPlan{};   // all of a sweep, or none
         if (!w.ok) continue;
         out.flops_per_amp.push_back(w.flops_per_amp);
         out.turned.push_back(w.turned);
+        out.n_acc.push_back(w.n_acc);
+        for (Gen::AdjOut& a : w.outs) {
+            for (auto& [acc, weight] : a.acc) acc += out.total_acc;
+            out.adj.push_back({a.slot, std::move(a.acc)});
+        }
+        out.acc0.push_back(out.total_acc);
+        out.total_acc += w.n_acc;
         const uint64_t sig = w.sig ^ (static_cast<uint64_t>(major) << 56) ^ (static_cast<uint64_t>(minor) << 48);
         out.idx[i] = static_cast<int>(sigs.size());
         sigs.push_back(sig);
@@ -1362,7 +1627,7 @@ JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int devic
             std::vector<double> coef;
             uint64_t sig = 0, turned = 0;
             Carry next;
-            gen_pass(*passes[i], plans[i], n, 0, true, f32, &srcs[j], &coef, &sig, &turned, nullptr,
+            gen_pass(*passes[i], plans[i], n, 0, true, f32, pair, &srcs[j], &coef, &sig, &turned, nullptr,
                      w.has_cin ? &w.cin : nullptr, w.final, w.final ? nullptr : &next);
             srcs[j] = std::string(kPrelude) + kPreludeDebug + srcs[j] + tag;
             char name[40];
@@ -1397,7 +1662,7 @@ JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int devic
             CUfunction f = nullptr;
             check_cu(drv.get_function(&f, mod, "qsv_jit_0"), "cuModuleGetFunction (JIT tiles)");
             check_cu(drv.set_attribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES,
-                                       static_cast<int>(jit_smem(f32))),
+                                       static_cast<int>(pair ? pair_smem(kPairMaxAcc) : jit_smem(f32))),
                      "cuFuncSetAttribute (JIT tiles)");
             g_kernels[{sigs[missing[j]], ctx}] = f;
         }
@@ -1406,27 +1671,98 @@ JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int devic
     return out;
 }
 
-void jit_launch(const JitPlan& plan, int pass, void* s, int n, cudaStream_t st) {
+namespace {
+void launch_pass(const JitPlan& plan, int pass, void* s, void* s2, double2* partials, int n, cudaStream_t st) {
     const int k = plan.idx.at(pass);
     if (k < 0) throw std::logic_error("JIT tiles: pass was not compiled");
     int sms = 0, device = 0;
     check_cuda(cudaGetDevice(&device), "device");
     check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "sm count");
     unsigned long long n_tiles = 1ull << (n - kRtQubits);
+    const int ctas = plan.pair ? 1 : jit_ctas(plan.f32);
     const unsigned grid = static_cast<unsigned>(
-        std::min<unsigned long long>(n_tiles, static_cast<unsigned long long>(jit_ctas(plan.f32)) * sms));
+        std::min<unsigned long long>(n_tiles, static_cast<unsigned long long>(ctas) * sms));
     const std::vector<uint8_t>& c = plan.coef[static_cast<size_t>(k)];
     unsigned long long turned = plan.turned[static_cast<size_t>(k)];
+    double2* part = partials ? partials + static_cast<size_t>(plan.acc0[static_cast<size_t>(k)]) * grid : nullptr;
+    std::vector<void*> args{&s, &n_tiles, &turned};
+    if (plan.pair) args.insert(args.end(), {static_cast<void*>(&s2), static_cast<void*>(&part)});
+    args.push_back(const_cast<uint8_t*>(c.data()));
 #ifdef QSV_DEBUG_BOUNDS
     unsigned long long* dbg = jit_fault_word(device);
-    void* args[] = {&s, &n_tiles, &turned, const_cast<uint8_t*>(c.data()), &dbg};
-#else
-    void* args[] = {&s, &n_tiles, &turned, const_cast<uint8_t*>(c.data())};
+    args.push_back(&dbg);
 #endif
+    const size_t smem = plan.pair ? pair_smem(plan.n_acc[static_cast<size_t>(k)]) : jit_smem(plan.f32);
     check_cu(driver().launch(static_cast<CUfunction>(plan.fns[static_cast<size_t>(k)]), grid, 1, 1, kJitThreads, 1, 1,
-                             static_cast<unsigned>(jit_smem(plan.f32)),
-                             reinterpret_cast<CUstream>(st), args, nullptr),
+                             static_cast<unsigned>(smem), reinterpret_cast<CUstream>(st), args.data(), nullptr),
              "cuLaunchKernel (JIT tiles)");
+}
+}  // namespace
+
+void jit_launch(const JitPlan& plan, int pass, void* s, int n, cudaStream_t st) {
+    launch_pass(plan, pass, s, nullptr, nullptr, n, st);
+}
+
+void jit_launch_pair(const JitPlan& plan, int pass, void* psi, void* phi, double2* partials, int n, cudaStream_t st) {
+    launch_pass(plan, pass, psi, phi, partials, n, st);
+}
+
+bool run_adjoint_compiled(const std::vector<Op>& ops, double2* psi, double2* phi, int n, double2* partials, unsigned nb,
+                          cudaStream_t st, const std::function<void(const Op&)>& stream_op, uint64_t* launches, int* n_acc,
+                          std::vector<JitPlan::Adj>* steps) {
+    if (ops.empty()) return true;
+    // a pass ends where its accumulators or its parameters would overflow (at most 32 doubles of phase
+    // table and ratio a step, or the step's matrix)
+    std::vector<TilePass> passes;
+    for (TilePass& p : plan_tiles(ops, n, kRtQubits, coalesced_low_qubits(16), kJitPlanSeeds)) {
+        if (p.tile_qubits.empty()) {
+            for (const Op& o : p.ops)
+                if (o.kind == OP_ADJ) return false;
+            passes.push_back(std::move(p));
+            continue;
+        }
+        TilePass cur;
+        int acc = 0;
+        size_t words = 0;
+        auto close = [&] {
+            if (cur.ops.empty()) return;
+            cur.tile_qubits = p.tile_qubits;
+            cur.low = p.low;
+            passes.push_back(std::move(cur));
+            cur = TilePass{};
+            acc = 0;
+            words = 0;
+        };
+        for (Op& o : p.ops) {
+            const int a = o.kind != OP_ADJ ? 0 : o.k == 1 ? 2 : 1;
+            const size_t w = 34 + 2 * o.m.size();
+            if (acc + a > kPairMaxAcc || words + w > kJitMaxCoefDoubles - 400) close();
+            acc += a;
+            words += w;
+            cur.ops.push_back(std::move(o));
+        }
+        close();
+    }
+    std::vector<const TilePass*> ptrs;
+    for (const TilePass& p : passes) ptrs.push_back(&p);
+    int device = 0;
+    check_cuda(cudaGetDevice(&device), "device");
+    JitPlan plan = jit_prepare(ptrs, n, device, false, true);
+    if (plan.idx.empty()) return false;
+    for (size_t i = 0; i < passes.size(); ++i) {
+        if (passes[i].tile_qubits.empty()) {
+            for (const Op& o : passes[i].ops) stream_op(o);
+            continue;
+        }
+        jit_launch_pair(plan, static_cast<int>(i), psi, phi, partials + static_cast<size_t>(*n_acc) * nb, n, st);
+        ++*launches;
+    }
+    for (JitPlan::Adj& a : plan.adj) {
+        for (auto& [acc, weight] : a.acc) acc += *n_acc;
+        steps->push_back(std::move(a));
+    }
+    *n_acc += plan.total_acc;
+    return true;
 }
 
 std::string jit_source_for_test(const std::vector<const TilePass*>& passes, int n, bool f32, size_t* n_kernels) {
@@ -1441,7 +1777,7 @@ std::string jit_source_for_test(const std::vector<const TilePass*>& passes, int 
         std::vector<double> coef;
         uint64_t sig = 0, turned = 0;
         Carry out;
-        if (!gen_pass(*passes[i], plans[i], n, next, true, f32, &ps, &coef, &sig, &turned, nullptr,
+        if (!gen_pass(*passes[i], plans[i], n, next, true, f32, false, &ps, &coef, &sig, &turned, nullptr,
                       w.has_cin ? &w.cin : nullptr, w.final, w.final ? nullptr : &out))
             continue;
         if (next > 0) {

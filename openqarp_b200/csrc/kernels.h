@@ -160,14 +160,28 @@ void run_tiled(const std::vector<TilePass>& passes, vec2_t<T>* s, int n, cudaStr
 // The register-tile passes of a stream compiled to straight-line kernels.
 struct JitPlan {
     bool f32 = false;                       // complex64 storage
+    bool pair = false;                      // psi and phi together (adjoint)
     std::vector<int> idx;                   // per pass: kernel index, -1 = not compiled
     std::vector<std::vector<uint8_t>> coef; // per kernel: its coefficients (kernel parameters)
     std::vector<void*> fns;                 // per kernel: the loaded function (CUfunction)
     std::vector<uint64_t> turned;           // per kernel: qubits whose bits the store flips (kernel parameter)
     std::vector<double> flops_per_amp;      // per kernel: FP64 operations per amplitude (FMA = 2)
+    // pair plans: accumulators per kernel and before it, and each adjoint step's Im <phi|G|psi> as a
+    // weighted sum of accumulators, by the step's slot
+    std::vector<int> n_acc, acc0;
+    int total_acc = 0;
+    struct Adj {
+        int slot;
+        std::vector<std::pair<int, double>> acc;
+    };
+    std::vector<Adj> adj;
 };
-JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int device, bool f32);
+// `pair`: passes of the adjoint's reverse sweep over psi and phi (complex128); then every tile pass
+// compiles, or the plan comes back empty (idx empty).
+JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int device, bool f32, bool pair = false);
 void jit_launch(const JitPlan& plan, int pass, void* s, int n, cudaStream_t st);
+// accumulator a's partial of block b goes to partials[a * grid + b].x, grid = adjoint_tile_grid(n, kRtQubits)
+void jit_launch_pair(const JitPlan& plan, int pass, void* psi, void* phi, double2* partials, int n, cudaStream_t st);
 // host-only helpers for plan inspection and tests (no device work)
 std::string jit_source_for_test(const std::vector<const TilePass*>& passes, int n, bool f32, size_t* n_kernels);
 std::vector<char> jit_compile_for_test(const std::string& src, int cc_major, int cc_minor);
@@ -184,6 +198,18 @@ void run_adjoint_tiled(const std::vector<Op>& ops, vec2_t<T>* psi, vec2_t<T>* ph
                        double* d_partials, unsigned nb, cudaStream_t st, Workspace& ws,
                        const std::function<void(const Op&)>& stream_op, uint64_t* launches,
                        std::vector<int>* slot_order = nullptr);
+// The same in compiled pair passes (complex128, kern_tile_jit.cu): accumulators from *n_acc on, partials
+// [accumulator][block] in .x, steps' weighted sums appended to `steps`.  False, having done nothing, when
+// a pass cannot be compiled.
+bool run_adjoint_compiled(const std::vector<Op>& ops, double2* psi, double2* phi, int n, double2* partials, unsigned nb,
+                          cudaStream_t st, const std::function<void(const Op&)>& stream_op, uint64_t* launches, int* n_acc,
+                          std::vector<JitPlan::Adj>* steps);
+// float registers keep the interpreter: their inner products are summed in FP64, which the compiled
+// passes would do in conversions
+inline bool run_adjoint_compiled(const std::vector<Op>&, float2*, float2*, int, double2*, unsigned, cudaStream_t,
+                                 const std::function<void(const Op&)>&, uint64_t*, int*, std::vector<JitPlan::Adj>*) {
+    return false;
+}
 
 // ---------------------------------------------------------------- register tiles (kern_tile_rt.cu)
 struct RtUpload {

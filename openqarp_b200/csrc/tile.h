@@ -82,7 +82,8 @@ static_assert(sizeof(RtLayout) == kRtQubits, "a layout names every local bit onc
 // (CZ-like, phase -1) whose conditions follow as RT_SIGN_ITEM records and whose flips are
 // applied in one pass over the registers.
 enum RtKind : uint8_t { RT_XPOSE = 1, RT_RELABEL, RT_DENSE, RT_DIAG, RT_PHASE, RT_CTRL1, RT_PAULI, RT_SCALE,
-                        RT_G1, RT_GL, RT_SIGNS, RT_SIGN_ITEM };
+                        RT_G1, RT_GL, RT_SIGNS, RT_SIGN_ITEM,
+                        RT_ADJ };   // a reverse step of the adjoint (compiled pair passes only)
 
 struct RtStep {
     RtKind kind = RT_SCALE;

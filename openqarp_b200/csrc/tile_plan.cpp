@@ -198,6 +198,7 @@ bool rt_capable(const Op& o, uint32_t mix) {
         case OP_DENSE: return o.k <= kRtMaxDense && o.ctrl == 0;
         case OP_CTRL1: case OP_SWAP: return true;
         case OP_PAULI_ROT: return __builtin_popcount(mix) <= kRtRegBits;
+        case OP_ADJ: return o.k <= 2;
         default: return false;
     }
 }
@@ -405,8 +406,8 @@ bool plan_rt(const TilePass& pass, RtPlan* out, int amp_bytes) {
                 RtStep st;
                 st.op = &o;
                 switch (o.kind) {
-                    case OP_DENSE:
-                        st.kind = RT_DENSE;
+                    case OP_DENSE: case OP_ADJ:
+                        st.kind = o.kind == OP_ADJ ? RT_ADJ : RT_DENSE;
                         st.slot_of.resize(o.k);
                         for (int b = 0; b < o.k; ++b) {
                             st.slot_of[b] = slot_of_bit(L, local_of[o.qubits[b]]);

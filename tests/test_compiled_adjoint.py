@@ -1,0 +1,83 @@
+"""The compiled reverse sweep (complex128, executor 3) against the CPU oracle: every differentiable gate,
+angles on both sides of a quarter turn, fixed gates of every form between them, parameters shared by
+several gates, checkpoint restarts, a block no tile holds, and more steps than one pass accumulates."""
+import numpy as np
+import pytest
+
+from openqarp_b200 import Command, GateType as G, Param, Register, circuits, ir, observable
+
+ONE = [G.Rx, G.Ry, G.Rz, G.P]
+TWO = [G.CRx, G.CRy, G.CRz, G.CP, G.RXX, G.RYY, G.RZZ]
+
+
+def _circuit(n, seed, count, n_params=24, wide=False):
+    rng = np.random.default_rng([n, seed])
+    out = []
+    for i in range(count):
+        q = [int(x) for x in rng.permutation(n)[:3]]
+        p = Param.linear(float(rng.choice([-1.5, 1.0, 2.0])), f"t{int(rng.integers(n_params))}", float(rng.uniform(-1, 1)))
+        pick = int(rng.integers(0, 12))
+        if pick < 5:
+            out.append(Command(ONE[pick % 4], (q[0],), (p,)))
+        elif pick < 7:
+            out.append(Command(TWO[int(rng.integers(7))], (q[0], q[1]), (p,)))
+        elif pick == 7:
+            out.append(Command([G.H, G.X, G.Y, G.S, G.T, G.SX][int(rng.integers(6))], (q[0],)))
+        elif pick == 8:
+            out.append(Command([G.CX, G.CZ, G.SWAP, G.CH][int(rng.integers(4))], (q[0], q[1])))
+        elif pick == 9:
+            out.append(Command([G.CCX, G.MCZ][int(rng.integers(2))], tuple(q)))
+        elif pick == 10:
+            out.append(Command(G.GPhase, (), (p,)))
+        else:
+            out.append(Command(G.Ry, (q[0],), (float(rng.uniform(-7, 7)),)))
+    if wide:
+        z = rng.standard_normal((64, 64)) + 1j * rng.standard_normal((64, 64))
+        out.insert(count // 2, ir.custom(tuple(int(x) for x in rng.permutation(n)[:6]), np.linalg.qr(z)[0]))
+    names = [f"t{k}" for k in range(n_params)]
+    return out, {k: float(v) for k, v in zip(names, rng.uniform(-4, 4, n_params))}, names
+
+
+def _check(restatement, n, cmds, vals, names, checkpoint=-1):
+    obs = circuits.tfim_chain(n) + circuits.random_pauli_sum(n, 12, seed=n, max_weight=3)
+    masks = observable.to_masks(obs, n)
+    stream = ir.pack(cmds, vals, names)
+    want_e, want_g = restatement.adjoint(stream, n, len(names), masks)
+    reg = Register(n)
+    reg.configure(1, 0, 3)
+    reg.set_checkpoint_interval(checkpoint)
+    e, g = reg.adjoint(stream, len(names), masks)
+    # sums of a few hundred steps' inner products, each below |H| ~ 40 with 1e-14 rounding
+    assert abs(e - want_e) < 1e-10
+    np.testing.assert_allclose(g, want_g, atol=1e-9)
+    # the sweep leaves the state uncomputed
+    psi = reg.get_state()
+    psi[0] -= 1.0
+    assert np.max(np.abs(psi)) < 1e-11
+    reg.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,seed,count", [(14, 1, 60), (14, 2, 200), (15, 3, 200), (17, 4, 120)])
+def test_random_circuits_match_oracle(restatement, n, seed, count):
+    _check(restatement, n, *_circuit(n, seed, count))
+
+
+@pytest.mark.gpu
+def test_checkpoints_and_wide_block(restatement):
+    cmds, vals, names = _circuit(14, 5, 160)
+    _check(restatement, 14, cmds, vals, names, checkpoint=45)
+    cmds, vals, names = _circuit(15, 6, 80, wide=True)
+    _check(restatement, 15, cmds, vals, names)
+
+
+@pytest.mark.gpu
+def test_ansatz_layers_and_many_steps_on_few_qubits(restatement):
+    cmds, vals, names = circuits.hea(16, 4, seed=3)
+    _check(restatement, 16, cmds, vals, names)
+    # 200 steps on four qubits: one tile's pass is cut where its accumulators end
+    rng = np.random.default_rng(9)
+    names = [f"t{k}" for k in range(200)]
+    cmds = [Command(ONE[int(rng.integers(4))], (int(rng.integers(4)),), (Param.symbol(nm),)) for nm in names]
+    cmds = [Command(G.H, (q,)) for q in range(14)] + cmds
+    _check(restatement, 14, cmds, {nm: float(v) for nm, v in zip(names, rng.uniform(-4, 4, 200))}, names)
