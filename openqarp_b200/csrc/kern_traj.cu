@@ -330,6 +330,153 @@ __global__ void __launch_bounds__(kTrThreads) k_tr_apply_2x2(vec2_t<T>* __restri
     (*QSV_DBG(p + (i0 | qb))) = mk<T>(static_cast<T>(y1r), static_cast<T>(y1i));
 }
 
+// ---- Kraus channels of up to four qubits at a time.  A channel whose operators' K^dag K are diagonal
+// (amplitude damping, phase damping, any with at most one entry a row and column) fires with
+// probabilities that follow from |a|^2 alone, and its chosen operator only weights the two halves.  So
+// for neighbouring channels on four qubits one read gives the 16 sums of |a|^2 by their bits, from
+// which the shot decides the four in order (the sums of the later ones reweighted by the operators
+// chosen), and one pass applies the four operators to 16 amplitudes a thread, with the next four
+// qubits' sums on its way.  One qubit at a time read the register twice and wrote it once per
+// channel: 16 qubits, 1024 shots, 128 channels 60 ms; @@KRAUS@@.
+constexpr int kKrausGroup = 4;
+constexpr int kKrausMinQubits = 12;        // a block's 4096 amplitudes belong to one shot
+struct KrausPass {
+    uint8_t pos[kKrausGroup];      // qubits to apply, ascending
+    uint8_t slot[kKrausGroup];     // channel k of the group acts on register bit slot[k]
+    uint8_t at[kKrausGroup];       // bit positions, within the group index, of the next sums' qubits
+    int32_t n_sum;                 // how many (0: no sums)
+};
+
+// Group index g names the amplitudes that differ in the MA applied qubits; bits 0..4 of g are the
+// lane, 5..7 the warp, then the thread's iterations and the block.
+template <typename T, int MA>
+__global__ void __launch_bounds__(kTrThreads) k_tr_kraus_pass(vec2_t<T>* __restrict__ s, int n,
+                                                             const __grid_constant__ KrausPass kp,
+                                                             const int8_t* __restrict__ act,
+                                                             const double* __restrict__ kmat,
+                                                             double* __restrict__ sums) {
+    constexpr int kIters = 16 >> MA;
+    __shared__ double part[kIters * kTrThreads];
+    const uint32_t tid = threadIdx.x;
+    const uint64_t per_shot = 1ull << (n - kTrChunkLog);
+    const uint64_t shot = blockIdx.x / per_shot, chunk = blockIdx.x % per_shot;
+    vec2_t<T>* p = s + (shot << n);
+    const int on = MA > 0 ? *QSV_DBG(act + shot) : 0;
+    uint32_t sum_bits = 0;
+    for (int k = 0; k < kp.n_sum; ++k) sum_bits |= 1u << kp.at[k];
+#pragma unroll 1
+    for (int it = 0; it < kIters; ++it) {
+        const uint64_t g = chunk * (4096u >> MA) + static_cast<uint32_t>(it) * kTrThreads + tid;
+        const uint64_t base = insert_zeros(g, kp.pos, MA);
+        double xr[1 << MA], xi[1 << MA];
+        uint64_t off[1 << MA];
+#pragma unroll
+        for (int r = 0; r < (1 << MA); ++r) {
+            off[r] = base;
+#pragma unroll
+            for (int k = 0; k < MA; ++k)
+                if ((r >> k) & 1) off[r] |= 1ull << kp.pos[k];
+            const vec2_t<T> v = *QSV_DBG(p + off[r]);
+            xr[r] = v.x;
+            xi[r] = v.y;
+        }
+        if (on) {
+#pragma unroll
+            for (int k = 0; k < MA; ++k) {
+                if (!((on >> k) & 1)) continue;
+                const double* m = QSV_DBG_N(kmat + (shot * kKrausGroup + k) * 8, 64);
+                const double k0 = m[0], k1 = m[1], k2 = m[2], k3 = m[3], k4 = m[4], k5 = m[5], k6 = m[6], k7 = m[7];
+#pragma unroll
+                for (int b = 0; b < MA; ++b) {      // slot[k] is uniform; register indices stay constant
+                    if (kp.slot[k] != b) continue;
+#pragma unroll
+                    for (int r = 0; r < (1 << MA); ++r) {
+                        if ((r >> b) & 1) continue;
+                        const int h = r | (1 << b);
+                        const double ar = xr[r], ai = xi[r], br = xr[h], bi = xi[h];
+                        const double y0r = (k0 * ar - k1 * ai) + (k2 * br - k3 * bi);
+                        const double y0i = (k0 * ai + k1 * ar) + (k2 * bi + k3 * br);
+                        const double y1r = (k4 * ar - k5 * ai) + (k6 * br - k7 * bi);
+                        const double y1i = (k4 * ai + k5 * ar) + (k6 * bi + k7 * br);
+                        // rounded to the register's precision after each operator
+                        xr[r] = static_cast<T>(y0r);
+                        xi[r] = static_cast<T>(y0i);
+                        xr[h] = static_cast<T>(y1r);
+                        xi[h] = static_cast<T>(y1i);
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < (1 << MA); ++r) *QSV_DBG(p + off[r]) = mk<T>(static_cast<T>(xr[r]), static_cast<T>(xi[r]));
+        }
+        if (kp.n_sum) {
+            double v = 0.0;
+#pragma unroll
+            for (int r = 0; r < (1 << MA); ++r) v += xr[r] * xr[r] + xi[r] * xi[r];
+#pragma unroll
+            for (int b = 0; b < 5; ++b)
+                if (!((sum_bits >> b) & 1u)) v += __shfl_xor_sync(0xffffffffu, v, 1 << b);
+            part[it * kTrThreads + tid] = v;
+        }
+    }
+    if (!kp.n_sum) return;
+    __syncthreads();
+    if (tid >= (1u << kp.n_sum)) return;
+    // sum `tid`: in every warp row whose bits match, the lane whose summed-over bits are 0
+    uint64_t want = 0;
+    for (int k = 0; k < kp.n_sum; ++k) want |= static_cast<uint64_t>((tid >> k) & 1u) << kp.at[k];
+    uint64_t mask = 0;
+    for (int k = 0; k < kp.n_sum; ++k) mask |= 1ull << kp.at[k];
+    const uint64_t high = mask & ~31ull;
+    double t = 0.0;
+    for (int w = 0; w < kIters * (kTrThreads / 32); ++w) {
+        const uint64_t g = chunk * (4096u >> MA) + static_cast<uint32_t>(w) * 32u;
+        if (((g ^ want) & high) == 0) t += part[w * 32 + static_cast<uint32_t>(want & mask & 31ull)];
+    }
+    *QSV_DBG(sums + (static_cast<uint64_t>(blockIdx.x) << kKrausGroup) + tid) = t;
+}
+
+// One thread per shot: the group's channels in order from the sums of |a|^2 by their qubits' bits.
+struct KrausChannels {
+    uint32_t poff[kKrausGroup];
+    int32_t n_ops[kKrausGroup];
+    int32_t count;
+};
+__global__ void k_tr_kraus_group(const uint8_t* __restrict__ pass, const double* __restrict__ sums, uint64_t per_shot,
+                                 MtState mt, int n_shots, const double* __restrict__ prm,
+                                 const __grid_constant__ KrausChannels ch, int8_t* __restrict__ act,
+                                 double* __restrict__ kmat) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n_shots) return;
+    *QSV_DBG(act + s) = 0;
+    if (!*QSV_DBG(pass + s)) return;
+    double w[1 << kKrausGroup];
+#pragma unroll
+    for (int b = 0; b < (1 << kKrausGroup); ++b) w[b] = 0.0;
+    for (uint64_t c = 0; c < per_shot; ++c)
+#pragma unroll
+        for (int b = 0; b < (1 << kKrausGroup); ++b)
+            if (b < (1 << ch.count)) w[b] += *QSV_DBG(sums + ((static_cast<uint64_t>(s) * per_shot + c) << kKrausGroup) + b);
+    int on = 0;
+    const MtView g = mt.of(s);
+#pragma unroll
+    for (int k = 0; k < kKrausGroup; ++k) {
+        if (k >= ch.count) break;
+        double r0 = 0.0, r1 = 0.0;
+#pragma unroll
+        for (int b = 0; b < (1 << kKrausGroup); ++b) (((b >> k) & 1) ? r1 : r0) += w[b];
+        double m[8];
+        if (!tr_choose_kraus(r0, r1, 0.0, 0.0, prm + ch.poff[k], ch.n_ops[k], g, m)) continue;
+        on |= 1 << k;
+        for (int e = 0; e < 8; ++e) *QSV_DBG(kmat + (static_cast<uint64_t>(s) * kKrausGroup + k) * 8 + e) = m[e];
+        const double w0 = m[0] * m[0] + m[1] * m[1] + m[4] * m[4] + m[5] * m[5];
+        const double w1 = m[2] * m[2] + m[3] * m[3] + m[6] * m[6] + m[7] * m[7];
+#pragma unroll
+        for (int b = 0; b < (1 << kKrausGroup); ++b) w[b] *= ((b >> k) & 1) ? w1 : w0;
+    }
+    *QSV_DBG(act + s) = static_cast<int8_t>(on);
+}
+
 // Projection and renormalisation on the pairs (i, i | 2^q) of every deciding shot; Reset moves
 // an outcome-1 survivor back to |0> (the X after the projection).
 template <typename T>
@@ -751,7 +898,8 @@ void run_trajectories(const std::vector<Cmd>& suffix, int n, int n_cbits, const 
 
     // batch size: a power of two, bounded by the shots and by the device memory budget
     const size_t state_bytes = sizeof(vec2_t<T>) << n;
-    const size_t per_shot_bytes = 8 * 18 + 4 * (kMtN + 3) + 2 + 8 * n_chunks + (plan.kraus ? 32 * n_pchunks : 0);
+    const size_t per_shot_bytes = 8 * (18 + 8 * (kKrausGroup - 1)) + 4 * (kMtN + 3) + 2 + 8 * n_chunks +
+                                  (plan.kraus ? std::max<size_t>(32 * n_pchunks, (8ull << kKrausGroup) * n_chunks) : 0);
     size_t free_b = 0, total_b = 0;
     check_cuda(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
     const size_t budget = (free_b + ws.traj_held()) / 2;   // buffers kept from an earlier run count as free
@@ -784,9 +932,10 @@ void run_trajectories(const std::vector<Cmd>& suffix, int n, int n_cbits, const 
     uint64_t* d_out = reinterpret_cast<uint64_t*>(carve(8 * B));
     uint64_t* d_ax = reinterpret_cast<uint64_t*>(carve(8 * B));
     uint64_t* d_az = reinterpret_cast<uint64_t*>(carve(8 * B));
-    double* d_kmat = reinterpret_cast<double*>(carve(8 * 8 * B));
+    double* d_kmat = reinterpret_cast<double*>(carve(8 * 8 * kKrausGroup * B));
     double* d_chunks = reinterpret_cast<double*>(carve(8 * B * n_chunks));
-    double* d_rho = plan.kraus ? reinterpret_cast<double*>(carve(32 * B * n_pchunks)) : nullptr;
+    double* d_rho = plan.kraus ? reinterpret_cast<double*>(carve(B * std::max<size_t>(32 * n_pchunks, (8ull << kKrausGroup) * n_chunks)))
+                               : nullptr;
     uint32_t* d_mt = reinterpret_cast<uint32_t*>(carve(4ull * kMtN * B));
     uint32_t* d_mtidx = reinterpret_cast<uint32_t*>(carve(4 * B));
     uint32_t* d_any = reinterpret_cast<uint32_t*>(carve(4 * B));
@@ -836,6 +985,26 @@ void run_trajectories(const std::vector<Cmd>& suffix, int n, int n_cbits, const 
         }
         group_len[i] = static_cast<uint32_t>(j - i);
         i = j;
+    }
+    // Kraus steps that follow one another with one guard, on distinct qubits, all with diagonal K^dag K:
+    // decided and applied four qubits at a time
+    auto diagonal_weights = [&](const TrStep& t) {
+        for (int o = 0; o < t.n_ops; ++o) {
+            const double* k = plan.noise_prm.data() + t.poff + 8 * o;
+            const c128 x = std::conj(c128(k[0], k[1])) * c128(k[2], k[3]) + std::conj(c128(k[4], k[5])) * c128(k[6], k[7]);
+            if (x != 0.0) return false;
+        }
+        return true;
+    };
+    std::vector<uint32_t> kraus_len(plan.steps.size(), 0);
+    for (size_t i = 0; i < plan.steps.size() && n >= kKrausMinQubits;) {
+        uint64_t used = 0;
+        size_t j = i;
+        while (j < plan.steps.size() && plan.steps[j].kind == TrStep::NOISE && plan.steps[j].noise == NOISE_KRAUS &&
+               plan.steps[j].g == plan.steps[i].g && !((used >> plan.steps[j].nq.q[0]) & 1) && diagonal_weights(plan.steps[j]))
+            used |= 1ull << plan.steps[j++].nq.q[0];
+        if (j > i) kraus_len[i] = static_cast<uint32_t>(j - i);
+        i = std::max(j, i + 1);
     }
     DeviceBuffer chan_buf(chans.size() * sizeof(TrChannelDev));
     TrChannelDev* d_chans = static_cast<TrChannelDev*>(chan_buf.p);
@@ -928,7 +1097,50 @@ void run_trajectories(const std::vector<Cmd>& suffix, int n, int n_cbits, const 
                     break;
                 case TrStep::NOISE: {
                     guard(step.g);
-                    if (step.noise == NOISE_KRAUS) {
+                    if (kraus_len[si]) {
+                        // groups [a, b): sums of the first, then (decide, apply with the next group's sums)
+                        const size_t end = si + kraus_len[si];
+                        auto pass_of = [&](size_t a, size_t b, size_t c) {   // apply [a, b), sums of [b, c)
+                            KrausPass kp{};
+                            uint64_t applied = 0;
+                            for (size_t i = a; i < b; ++i) applied |= 1ull << plan.steps[i].nq.q[0];
+                            int at = 0;
+                            for (int q = 0; q < n; ++q)
+                                if ((applied >> q) & 1) kp.pos[at++] = static_cast<uint8_t>(q);
+                            for (size_t i = a; i < b; ++i)
+                                kp.slot[i - a] = static_cast<uint8_t>(__builtin_popcountll(applied & ((1ull << plan.steps[i].nq.q[0]) - 1)));
+                            kp.n_sum = static_cast<int32_t>(c - b);
+                            for (size_t i = b; i < c; ++i) {
+                                const int q = plan.steps[i].nq.q[0];
+                                kp.at[i - b] = static_cast<uint8_t>(q - __builtin_popcountll(applied & ((1ull << q) - 1)));
+                            }
+                            const unsigned grid = static_cast<unsigned>(static_cast<uint64_t>(nb) << (n - kTrChunkLog));
+                            switch (b - a) {
+                                case 0: k_tr_kraus_pass<T, 0><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                                case 1: k_tr_kraus_pass<T, 1><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                                case 2: k_tr_kraus_pass<T, 2><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                                case 3: k_tr_kraus_pass<T, 3><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                                default: k_tr_kraus_pass<T, 4><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                            }
+                            n_launch++;
+                        };
+                        auto cut = [&](size_t i) { return std::min(end, i + kKrausGroup); };
+                        pass_of(si, si, cut(si));
+                        for (size_t a = si; a < end; a = cut(a)) {
+                            const size_t b = cut(a);
+                            KrausChannels kc{};
+                            kc.count = static_cast<int32_t>(b - a);
+                            for (size_t i = a; i < b; ++i) {
+                                kc.poff[i - a] = static_cast<uint32_t>(plan.steps[i].poff);
+                                kc.n_ops[i - a] = plan.steps[i].n_ops;
+                            }
+                            k_tr_kraus_group<<<static_cast<unsigned>(nb + 63) / 64, 64, 0, st>>>(d_pass, d_rho, n_chunks, mt, nb, d_nprm, kc,
+                                                                                d_outcome, d_kmat);
+                            n_launch++;
+                            pass_of(a, b, cut(b));
+                        }
+                        si = end - 1;
+                    } else if (step.noise == NOISE_KRAUS) {
                         const int q = step.nq.q[0];
                         k_tr_rho_chunks<T><<<static_cast<unsigned>(nb * n_pchunks), kTrThreads, 0, st>>>(s, n, q,
                                                                                                       d_rho);
