@@ -337,12 +337,15 @@ __global__ void __launch_bounds__(kTrThreads) k_tr_apply_2x2(vec2_t<T>* __restri
 // which the shot decides the four in order (the sums of the later ones reweighted by the operators
 // chosen), and one pass applies the four operators to 16 amplitudes a thread, with the next four
 // qubits' sums on its way.  One qubit at a time read the register twice and wrote it once per
-// channel: 16 qubits, 1024 shots, 128 channels 60 ms; @@KRAUS@@.
+// channel: 16 qubits, 1024 shots, 128 channels 60 ms; 17 ms so.  A pass takes 0.43 ms of 2 GiB moved
+// (0.70 where the four qubits include the lowest, whose 16-byte runs do not coalesce).  Measurements
+// that follow one another are the same with projectors (16 final ones 6.2 -> 2.2 ms).
 constexpr int kKrausGroup = 4;
 constexpr int kKrausMinQubits = 12;        // a block's 4096 amplitudes belong to one shot
+constexpr int kKrausMaxQubits = 31;        // 32-bit indices within a shot
 struct KrausPass {
     uint8_t pos[kKrausGroup];      // qubits to apply, ascending
-    uint8_t slot[kKrausGroup];     // channel k of the group acts on register bit slot[k]
+    uint32_t off[1 << kKrausGroup];   // index bits of register r: channel k acts on register bit k
     uint8_t at[kKrausGroup];       // bit positions, within the group index, of the next sums' qubits
     int32_t n_sum;                 // how many (0: no sums)
 };
@@ -350,7 +353,7 @@ struct KrausPass {
 // Group index g names the amplitudes that differ in the MA applied qubits; bits 0..4 of g are the
 // lane, 5..7 the warp, then the thread's iterations and the block.
 template <typename T, int MA>
-__global__ void __launch_bounds__(kTrThreads) k_tr_kraus_pass(vec2_t<T>* __restrict__ s, int n,
+__global__ void __launch_bounds__(kTrThreads, 2) k_tr_kraus_pass(vec2_t<T>* __restrict__ s, int n,
                                                              const __grid_constant__ KrausPass kp,
                                                              const int8_t* __restrict__ act,
                                                              const double* __restrict__ kmat,
@@ -367,16 +370,11 @@ __global__ void __launch_bounds__(kTrThreads) k_tr_kraus_pass(vec2_t<T>* __restr
 #pragma unroll 1
     for (int it = 0; it < kIters; ++it) {
         const uint64_t g = chunk * (4096u >> MA) + static_cast<uint32_t>(it) * kTrThreads + tid;
-        const uint64_t base = insert_zeros(g, kp.pos, MA);
+        const uint32_t base = static_cast<uint32_t>(insert_zeros(g, kp.pos, MA));
         double xr[1 << MA], xi[1 << MA];
-        uint64_t off[1 << MA];
 #pragma unroll
         for (int r = 0; r < (1 << MA); ++r) {
-            off[r] = base;
-#pragma unroll
-            for (int k = 0; k < MA; ++k)
-                if ((r >> k) & 1) off[r] |= 1ull << kp.pos[k];
-            const vec2_t<T> v = *QSV_DBG(p + off[r]);
+            const vec2_t<T> v = *QSV_DBG(p + (base | kp.off[r]));
             xr[r] = v.x;
             xi[r] = v.y;
         }
@@ -387,27 +385,23 @@ __global__ void __launch_bounds__(kTrThreads) k_tr_kraus_pass(vec2_t<T>* __restr
                 const double* m = QSV_DBG_N(kmat + (shot * kKrausGroup + k) * 8, 64);
                 const double k0 = m[0], k1 = m[1], k2 = m[2], k3 = m[3], k4 = m[4], k5 = m[5], k6 = m[6], k7 = m[7];
 #pragma unroll
-                for (int b = 0; b < MA; ++b) {      // slot[k] is uniform; register indices stay constant
-                    if (kp.slot[k] != b) continue;
-#pragma unroll
-                    for (int r = 0; r < (1 << MA); ++r) {
-                        if ((r >> b) & 1) continue;
-                        const int h = r | (1 << b);
-                        const double ar = xr[r], ai = xi[r], br = xr[h], bi = xi[h];
-                        const double y0r = (k0 * ar - k1 * ai) + (k2 * br - k3 * bi);
-                        const double y0i = (k0 * ai + k1 * ar) + (k2 * bi + k3 * br);
-                        const double y1r = (k4 * ar - k5 * ai) + (k6 * br - k7 * bi);
-                        const double y1i = (k4 * ai + k5 * ar) + (k6 * bi + k7 * br);
-                        // rounded to the register's precision after each operator
-                        xr[r] = static_cast<T>(y0r);
-                        xi[r] = static_cast<T>(y0i);
-                        xr[h] = static_cast<T>(y1r);
-                        xi[h] = static_cast<T>(y1i);
-                    }
+                for (int r = 0; r < (1 << MA); ++r) {
+                    if ((r >> k) & 1) continue;
+                    const int h = r | (1 << k);
+                    const double ar = xr[r], ai = xi[r], br = xr[h], bi = xi[h];
+                    const double y0r = (k0 * ar - k1 * ai) + (k2 * br - k3 * bi);
+                    const double y0i = (k0 * ai + k1 * ar) + (k2 * bi + k3 * br);
+                    const double y1r = (k4 * ar - k5 * ai) + (k6 * br - k7 * bi);
+                    const double y1i = (k4 * ai + k5 * ar) + (k6 * bi + k7 * br);
+                    // rounded to the register's precision after each operator
+                    xr[r] = static_cast<T>(y0r);
+                    xi[r] = static_cast<T>(y0i);
+                    xr[h] = static_cast<T>(y1r);
+                    xi[h] = static_cast<T>(y1i);
                 }
             }
 #pragma unroll
-            for (int r = 0; r < (1 << MA); ++r) *QSV_DBG(p + off[r]) = mk<T>(static_cast<T>(xr[r]), static_cast<T>(xi[r]));
+            for (int r = 0; r < (1 << MA); ++r) *QSV_DBG(p + (base | kp.off[r])) = mk<T>(static_cast<T>(xr[r]), static_cast<T>(xi[r]));
         }
         if (kp.n_sum) {
             double v = 0.0;
@@ -436,45 +430,69 @@ __global__ void __launch_bounds__(kTrThreads) k_tr_kraus_pass(vec2_t<T>* __restr
     *QSV_DBG(sums + (static_cast<uint64_t>(blockIdx.x) << kKrausGroup) + tid) = t;
 }
 
-// One thread per shot: the group's channels in order from the sums of |a|^2 by their qubits' bits.
+// Sixteen lanes a shot, lane b holding the sum whose qubits' bits are b; lane 0 draws.  The group's steps
+// in order: Kraus channels, or measurements into cbits (operators diag(scale, 0) or diag(0, scale)).
 struct KrausChannels {
     uint32_t poff[kKrausGroup];
-    int32_t n_ops[kKrausGroup];
+    int32_t n_ops[kKrausGroup];    // Kraus operators; 0: a measurement
+    int32_t cbit[kKrausGroup];     // measurements: -1 not recorded
     int32_t count;
 };
-__global__ void k_tr_kraus_group(const uint8_t* __restrict__ pass, const double* __restrict__ sums, uint64_t per_shot,
-                                 MtState mt, int n_shots, const double* __restrict__ prm,
-                                 const __grid_constant__ KrausChannels ch, int8_t* __restrict__ act,
-                                 double* __restrict__ kmat) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(64) k_tr_kraus_group(const uint8_t* __restrict__ pass, const double* __restrict__ sums,
+                                                       uint64_t per_shot, MtState mt, int n_shots, const double* __restrict__ prm,
+                                                       const __grid_constant__ KrausChannels ch, int8_t* __restrict__ act,
+                                                       double* __restrict__ kmat, uint64_t* __restrict__ cbits) {
+    const int s = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> kKrausGroup);
+    const unsigned lane = threadIdx.x & 15u, half = 0xffffu << (threadIdx.x & 16u);
     if (s >= n_shots) return;
-    *QSV_DBG(act + s) = 0;
-    if (!*QSV_DBG(pass + s)) return;
-    double w[1 << kKrausGroup];
-#pragma unroll
-    for (int b = 0; b < (1 << kKrausGroup); ++b) w[b] = 0.0;
-    for (uint64_t c = 0; c < per_shot; ++c)
-#pragma unroll
-        for (int b = 0; b < (1 << kKrausGroup); ++b)
-            if (b < (1 << ch.count)) w[b] += *QSV_DBG(sums + ((static_cast<uint64_t>(s) * per_shot + c) << kKrausGroup) + b);
+    if (!*QSV_DBG(pass + s)) {
+        if (lane == 0) *QSV_DBG(act + s) = 0;
+        return;
+    }
+    double w = 0.0;
+    if (lane < (1u << ch.count))
+        for (uint64_t c = 0; c < per_shot; ++c) w += *QSV_DBG(sums + ((static_cast<uint64_t>(s) * per_shot + c) << kKrausGroup) + lane);
     int on = 0;
     const MtView g = mt.of(s);
 #pragma unroll
     for (int k = 0; k < kKrausGroup; ++k) {
         if (k >= ch.count) break;
-        double r0 = 0.0, r1 = 0.0;
+        const bool up = (lane >> k) & 1u;
+        double r0 = up ? 0.0 : w, r1 = up ? w : 0.0;
 #pragma unroll
-        for (int b = 0; b < (1 << kKrausGroup); ++b) (((b >> k) & 1) ? r1 : r0) += w[b];
-        double m[8];
-        if (!tr_choose_kraus(r0, r1, 0.0, 0.0, prm + ch.poff[k], ch.n_ops[k], g, m)) continue;
-        on |= 1 << k;
-        for (int e = 0; e < 8; ++e) *QSV_DBG(kmat + (static_cast<uint64_t>(s) * kKrausGroup + k) * 8 + e) = m[e];
-        const double w0 = m[0] * m[0] + m[1] * m[1] + m[4] * m[4] + m[5] * m[5];
-        const double w1 = m[2] * m[2] + m[3] * m[3] + m[6] * m[6] + m[7] * m[7];
-#pragma unroll
-        for (int b = 0; b < (1 << kKrausGroup); ++b) w[b] *= ((b >> k) & 1) ? w1 : w0;
+        for (int o = 1; o < 16; o <<= 1) {
+            r0 += __shfl_xor_sync(half, r0, o, 16);
+            r1 += __shfl_xor_sync(half, r1, o, 16);
+        }
+        double w0 = 1.0, w1 = 1.0;
+        if (lane == 0) {
+            double m[8];
+            bool fires = true;
+            if (ch.n_ops[k]) {
+                fires = tr_choose_kraus(r0, r1, 0.0, 0.0, prm + ch.poff[k], ch.n_ops[k], g, m);
+            } else {
+                double scale;
+                const bool one = tr_decide(r0, g, &scale);
+                for (int e = 0; e < 8; ++e) m[e] = 0.0;
+                m[one ? 6 : 0] = scale;
+                if (ch.cbit[k] >= 0) {
+                    const uint64_t bit = 1ull << ch.cbit[k];
+                    uint64_t* cb = QSV_DBG(cbits + s);
+                    *cb = one ? *cb | bit : *cb & ~bit;
+                }
+            }
+            if (fires) {
+                on |= 1 << k;
+                for (int e = 0; e < 8; ++e) *QSV_DBG(kmat + (static_cast<uint64_t>(s) * kKrausGroup + k) * 8 + e) = m[e];
+                w0 = m[0] * m[0] + m[1] * m[1] + m[4] * m[4] + m[5] * m[5];
+                w1 = m[2] * m[2] + m[3] * m[3] + m[6] * m[6] + m[7] * m[7];
+            }
+        }
+        w0 = __shfl_sync(half, w0, 0, 16);
+        w1 = __shfl_sync(half, w1, 0, 16);
+        w *= up ? w1 : w0;
     }
-    *QSV_DBG(act + s) = static_cast<int8_t>(on);
+    if (lane == 0) *QSV_DBG(act + s) = static_cast<int8_t>(on);
 }
 
 // Projection and renormalisation on the pairs (i, i | 2^q) of every deciding shot; Reset moves
@@ -680,6 +698,7 @@ TrPlan build_plan(const std::vector<Cmd>& suffix, int n, int n_cbits, int fusion
             st.kind = TrStep::OPS;
             for (const Cmd& c : fuse_for_dispatch(cmds, n, fusion_max, fusion_min))
                 for (Op& o : lower(c, n)) st.ops.push_back(std::move(o));
+            st.cmds = std::move(cmds);
             if (!st.ops.empty()) plan.steps.push_back(std::move(st));
             return;
         }
@@ -898,8 +917,9 @@ void run_trajectories(const std::vector<Cmd>& suffix, int n, int n_cbits, const 
 
     // batch size: a power of two, bounded by the shots and by the device memory budget
     const size_t state_bytes = sizeof(vec2_t<T>) << n;
+    const size_t rho_bytes = std::max<size_t>(plan.kraus ? 32 * n_pchunks : 0, n >= kKrausMinQubits ? (8ull << kKrausGroup) * n_chunks : 0);
     const size_t per_shot_bytes = 8 * (18 + 8 * (kKrausGroup - 1)) + 4 * (kMtN + 3) + 2 + 8 * n_chunks +
-                                  (plan.kraus ? std::max<size_t>(32 * n_pchunks, (8ull << kKrausGroup) * n_chunks) : 0);
+                                  rho_bytes;
     size_t free_b = 0, total_b = 0;
     check_cuda(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
     const size_t budget = (free_b + ws.traj_held()) / 2;   // buffers kept from an earlier run count as free
@@ -934,8 +954,7 @@ void run_trajectories(const std::vector<Cmd>& suffix, int n, int n_cbits, const 
     uint64_t* d_az = reinterpret_cast<uint64_t*>(carve(8 * B));
     double* d_kmat = reinterpret_cast<double*>(carve(8 * 8 * kKrausGroup * B));
     double* d_chunks = reinterpret_cast<double*>(carve(8 * B * n_chunks));
-    double* d_rho = plan.kraus ? reinterpret_cast<double*>(carve(B * std::max<size_t>(32 * n_pchunks, (8ull << kKrausGroup) * n_chunks)))
-                               : nullptr;
+    double* d_rho = reinterpret_cast<double*>(carve(rho_bytes * B));
     uint32_t* d_mt = reinterpret_cast<uint32_t*>(carve(4ull * kMtN * B));
     uint32_t* d_mtidx = reinterpret_cast<uint32_t*>(carve(4 * B));
     uint32_t* d_any = reinterpret_cast<uint32_t*>(carve(4 * B));
@@ -986,9 +1005,12 @@ void run_trajectories(const std::vector<Cmd>& suffix, int n, int n_cbits, const 
         group_len[i] = static_cast<uint32_t>(j - i);
         i = j;
     }
-    // Kraus steps that follow one another with one guard, on distinct qubits, all with diagonal K^dag K:
-    // decided and applied four qubits at a time
+    // Kraus steps with diagonal K^dag K, and measurements, that follow one another with one guard on
+    // distinct qubits: decided and applied four qubits at a time.  (A lone measurement keeps its own
+    // kernels: they read one half of the register and move no zeros.)
     auto diagonal_weights = [&](const TrStep& t) {
+        if (t.kind == TrStep::MEASURE) return !t.reset;
+        if (t.kind != TrStep::NOISE || t.noise != NOISE_KRAUS) return false;
         for (int o = 0; o < t.n_ops; ++o) {
             const double* k = plan.noise_prm.data() + t.poff + 8 * o;
             const c128 x = std::conj(c128(k[0], k[1])) * c128(k[2], k[3]) + std::conj(c128(k[4], k[5])) * c128(k[6], k[7]);
@@ -996,14 +1018,18 @@ void run_trajectories(const std::vector<Cmd>& suffix, int n, int n_cbits, const 
         }
         return true;
     };
+    auto qubit_of = [](const TrStep& t) { return t.kind == TrStep::MEASURE ? t.qubit : static_cast<int>(t.nq.q[0]); };
+    // a measurement whose cbit its own guard reads changes what the next one's guard sees
+    auto writes_condition = [](const TrStep& t) { return t.cbit >= 0 && ((t.g.cmask >> t.cbit) & 1); };
     std::vector<uint32_t> kraus_len(plan.steps.size(), 0);
-    for (size_t i = 0; i < plan.steps.size() && n >= kKrausMinQubits;) {
+    for (size_t i = 0; i < plan.steps.size() && n >= kKrausMinQubits && n <= kKrausMaxQubits;) {
         uint64_t used = 0;
         size_t j = i;
-        while (j < plan.steps.size() && plan.steps[j].kind == TrStep::NOISE && plan.steps[j].noise == NOISE_KRAUS &&
-               plan.steps[j].g == plan.steps[i].g && !((used >> plan.steps[j].nq.q[0]) & 1) && diagonal_weights(plan.steps[j]))
-            used |= 1ull << plan.steps[j++].nq.q[0];
-        if (j > i) kraus_len[i] = static_cast<uint32_t>(j - i);
+        while (j < plan.steps.size() && plan.steps[j].g == plan.steps[i].g && !((used >> qubit_of(plan.steps[j])) & 1) &&
+               diagonal_weights(plan.steps[j]) && plan.steps[j].kind == plan.steps[i].kind &&
+               (plan.steps[j].kind != TrStep::MEASURE || !writes_condition(plan.steps[j])))
+            used |= 1ull << qubit_of(plan.steps[j++]);
+        if (j > i + (plan.steps[i].kind == TrStep::MEASURE ? 1 : 0)) kraus_len[i] = static_cast<uint32_t>(j - i);
         i = std::max(j, i + 1);
     }
     DeviceBuffer chan_buf(chans.size() * sizeof(TrChannelDev));
@@ -1036,10 +1062,78 @@ void run_trajectories(const std::vector<Cmd>& suffix, int n, int n_cbits, const 
                                                               g.cmask, g.cwant);
             n_launch++;
         };
+        // A segment of one-qubit layers and pairs of a complex128 batch beyond L2 takes register-tile
+        // passes (one-qubit fusion) where one does the work of three or more stream passes: 26 qubits,
+        // a tile pass 0.87 ms against 0.17 to 0.31 ms an op; 16 noisy qubits, 1024 shots, 31 -> 21 ms.
+        auto tile_ops_now = [&](const TrStep& step) {
+            constexpr int kTileWide = 22;
+            if (sizeof(T) != sizeof(double) || nw < kTileWide || step.ops.size() < 3) return false;
+            std::vector<Op> ops;
+            for (const Cmd& c : fuse_for_dispatch(step.cmds, n, 1, opt.fusion_min))
+                for (Op& o : lower(c, n)) ops.push_back(std::move(o));
+            const std::vector<TilePass> passes = plan_tiles(ops, nw, kRtQubits, kTileLowQubits);
+            if (3 * passes.size() > step.ops.size()) return false;
+            run_tiled<T>(passes, s, nw, st, ws, [&](const Op& o) { launch_op<T>(o, s, nw, st, ws); }, true, false);
+            n_launch += passes.size();
+            return true;
+        };
+        auto run_group = [&](size_t si) {
+            guard(plan.steps[si].g);
+            // groups [a, b): sums of the first, then (decide, apply with the next group's sums)
+            const size_t end = si + kraus_len[si];
+            auto pass_of = [&](size_t a, size_t b, size_t c) {   // apply [a, b), sums of [b, c)
+                KrausPass kp{};
+                uint64_t applied = 0;
+                for (size_t i = a; i < b; ++i) applied |= 1ull << qubit_of(plan.steps[i]);
+                int at = 0;
+                for (int q = 0; q < n; ++q)
+                    if ((applied >> q) & 1) kp.pos[at++] = static_cast<uint8_t>(q);
+                for (uint32_t r = 0; r < (1u << (b - a)); ++r)
+                    for (size_t i = a; i < b; ++i)
+                        if ((r >> (i - a)) & 1) kp.off[r] |= 1u << qubit_of(plan.steps[i]);
+                kp.n_sum = static_cast<int32_t>(c - b);
+                for (size_t i = b; i < c; ++i) {
+                    const int q = qubit_of(plan.steps[i]);
+                    kp.at[i - b] = static_cast<uint8_t>(q - __builtin_popcountll(applied & ((1ull << q) - 1)));
+                }
+                const unsigned grid = static_cast<unsigned>(static_cast<uint64_t>(nb) << (n - kTrChunkLog));
+                switch (b - a) {
+                    case 0: k_tr_kraus_pass<T, 0><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                    case 1: k_tr_kraus_pass<T, 1><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                    case 2: k_tr_kraus_pass<T, 2><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                    case 3: k_tr_kraus_pass<T, 3><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                    default: k_tr_kraus_pass<T, 4><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                }
+                n_launch++;
+            };
+            auto cut = [&](size_t i) { return std::min(end, i + kKrausGroup); };
+            pass_of(si, si, cut(si));
+            for (size_t a = si; a < end; a = cut(a)) {
+                const size_t b = cut(a);
+                KrausChannels kc{};
+                kc.count = static_cast<int32_t>(b - a);
+                for (size_t i = a; i < b; ++i) {
+                    kc.poff[i - a] = static_cast<uint32_t>(plan.steps[i].poff);
+                    kc.n_ops[i - a] = plan.steps[i].kind == TrStep::MEASURE ? 0 : plan.steps[i].n_ops;
+                    kc.cbit[i - a] = plan.steps[i].cbit;
+                }
+                k_tr_kraus_group<<<(static_cast<unsigned>(nb) * 16 + 63) / 64, 64, 0, st>>>(d_pass, d_rho, n_chunks, mt, nb, d_nprm,
+                                                                                            kc, d_outcome, d_kmat, d_cbits);
+                n_launch++;
+                pass_of(a, b, cut(b));
+            }
+        };
         for (size_t si = 0; si < plan.steps.size(); ++si) {
             const TrStep& step = plan.steps[si];
+            if (kraus_len[si]) {
+                run_group(si);
+                check_cuda(cudaGetLastError(), "trajectory step");
+                si += kraus_len[si] - 1;
+                continue;
+            }
             switch (step.kind) {
                 case TrStep::OPS:
+                    if (tile_ops_now(step)) break;
                     for (const Op& o : step.ops) {
                         launch_op<T>(o, s, nw, st, ws);
                         n_launch++;
@@ -1097,50 +1191,7 @@ void run_trajectories(const std::vector<Cmd>& suffix, int n, int n_cbits, const 
                     break;
                 case TrStep::NOISE: {
                     guard(step.g);
-                    if (kraus_len[si]) {
-                        // groups [a, b): sums of the first, then (decide, apply with the next group's sums)
-                        const size_t end = si + kraus_len[si];
-                        auto pass_of = [&](size_t a, size_t b, size_t c) {   // apply [a, b), sums of [b, c)
-                            KrausPass kp{};
-                            uint64_t applied = 0;
-                            for (size_t i = a; i < b; ++i) applied |= 1ull << plan.steps[i].nq.q[0];
-                            int at = 0;
-                            for (int q = 0; q < n; ++q)
-                                if ((applied >> q) & 1) kp.pos[at++] = static_cast<uint8_t>(q);
-                            for (size_t i = a; i < b; ++i)
-                                kp.slot[i - a] = static_cast<uint8_t>(__builtin_popcountll(applied & ((1ull << plan.steps[i].nq.q[0]) - 1)));
-                            kp.n_sum = static_cast<int32_t>(c - b);
-                            for (size_t i = b; i < c; ++i) {
-                                const int q = plan.steps[i].nq.q[0];
-                                kp.at[i - b] = static_cast<uint8_t>(q - __builtin_popcountll(applied & ((1ull << q) - 1)));
-                            }
-                            const unsigned grid = static_cast<unsigned>(static_cast<uint64_t>(nb) << (n - kTrChunkLog));
-                            switch (b - a) {
-                                case 0: k_tr_kraus_pass<T, 0><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
-                                case 1: k_tr_kraus_pass<T, 1><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
-                                case 2: k_tr_kraus_pass<T, 2><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
-                                case 3: k_tr_kraus_pass<T, 3><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
-                                default: k_tr_kraus_pass<T, 4><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
-                            }
-                            n_launch++;
-                        };
-                        auto cut = [&](size_t i) { return std::min(end, i + kKrausGroup); };
-                        pass_of(si, si, cut(si));
-                        for (size_t a = si; a < end; a = cut(a)) {
-                            const size_t b = cut(a);
-                            KrausChannels kc{};
-                            kc.count = static_cast<int32_t>(b - a);
-                            for (size_t i = a; i < b; ++i) {
-                                kc.poff[i - a] = static_cast<uint32_t>(plan.steps[i].poff);
-                                kc.n_ops[i - a] = plan.steps[i].n_ops;
-                            }
-                            k_tr_kraus_group<<<static_cast<unsigned>(nb + 63) / 64, 64, 0, st>>>(d_pass, d_rho, n_chunks, mt, nb, d_nprm, kc,
-                                                                                d_outcome, d_kmat);
-                            n_launch++;
-                            pass_of(a, b, cut(b));
-                        }
-                        si = end - 1;
-                    } else if (step.noise == NOISE_KRAUS) {
+                    if (step.noise == NOISE_KRAUS) {
                         const int q = step.nq.q[0];
                         k_tr_rho_chunks<T><<<static_cast<unsigned>(nb * n_pchunks), kTrThreads, 0, st>>>(s, n, q,
                                                                                                       d_rho);

@@ -39,6 +39,7 @@ struct TrStep {
     enum Kind { OPS, MDENSE, MSCALE, MOPS, MEASURE, BRANCH, NOISE } kind = OPS;
     TrGuard g;
     std::vector<Op> ops;          // OPS: every shot; MOPS: every shot, failing shots restored
+    std::vector<Cmd> cmds;        // OPS: the segment's commands, for tile passes
     int k = 0;                    // MDENSE width
     size_t moff = 0;              // MDENSE: first entry in the matrix table
     TrDenseArgs args{};           // MDENSE
