@@ -169,6 +169,8 @@ QSV_API int qsv_set_checkpoint_interval(void* h, int k);
 
 /* Register <- |0...0>. */
 QSV_API int qsv_reset(void* h);
+/* The same in stream order, without waiting for it. */
+QSV_API int qsv_reset_async(void* h);
 /* Register <- caller amplitudes (interleaved c128, len = 2^n).  validate != 0 checks
  * the norm within 1e-10 exactly as validate_initial_state (qarp_simulator.cpp:731-746). */
 QSV_API int qsv_set_state(void* h, const double* amps, uint64_t len, int validate);

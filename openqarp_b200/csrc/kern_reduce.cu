@@ -398,6 +398,11 @@ __global__ void k_scale_real(vec2_t<T>* __restrict__ s, uint64_t dim, double f) 
     }
 }
 
+template <typename T>
+__global__ void k_set_first(vec2_t<T>* __restrict__ s) {
+    *QSV_DBG(s) = mk<T>(T(1), T(0));
+}
+
 TermPtrs upload_terms(const PauliTerms& t, cudaStream_t st, Workspace& ws) {
     const size_t ng = t.gx.size(), nt = t.z.size();
     const size_t bytes = 8 * ng + 4 * (ng + 1) + 8 * nt + 16 * nt + 4 * 9 * ng + 64;
@@ -891,7 +896,15 @@ void reduce_slots(const double* d_partials, int n_slots, unsigned nb, cudaStream
     std::memcpy(out.data(), h, 2 * sizeof(double) * n_slots);
 }
 
+template <typename T>
+void set_first(vec2_t<T>* s, cudaStream_t st) {
+    k_set_first<T><<<1, 1, 0, st>>>(s);
+    check_cuda(cudaGetLastError(), "reset launch");
+}
+
 // explicit instantiations
+template void set_first<double>(double2*, cudaStream_t);
+template void set_first<float>(float2*, cudaStream_t);
 template void transition<double>(const double2*, const double2*, int, const PauliTerms&, cudaStream_t, Workspace&, double*);
 template void transition<float>(const float2*, const float2*, int, const PauliTerms&, cudaStream_t, Workspace&, double*);
 template void apply_observable<double>(const double2*, double2*, int, const PauliTerms&, cudaStream_t, Workspace&);

@@ -278,6 +278,9 @@ double norm2(const vec2_t<T>* s, int n, cudaStream_t st, Workspace& ws);
 template <typename TA, typename TB>
 void inner(const vec2_t<TA>* a, const vec2_t<TB>* b, int n, cudaStream_t st, Workspace& ws,
            double out[2]);
+// s[0] = 1
+template <typename T>
+void set_first(vec2_t<T>* s, cudaStream_t st);
 template <typename T>
 void scale_real(vec2_t<T>* s, int n, double f, cudaStream_t st);
 

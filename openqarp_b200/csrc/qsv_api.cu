@@ -567,14 +567,20 @@ int qsv_set_tile_qubits(void* hp, int m) {
     });
 }
 
-int qsv_reset(void* hp) {
+int qsv_reset_async(void* hp) {
     return guarded([&] {
         Handle* h = H_(hp);
+        // the first amplitude from a kernel: a copy from pageable memory would wait for the stream
         check_cuda(cudaMemsetAsync(h->state, 0, h->dim() * h->amp_bytes(), h->stream), "memset");
-        const double one[2] = {1.0, 0.0};
-        const float onef[2] = {1.0f, 0.0f};
-        check_cuda(cudaMemcpyAsync(h->state, h->dtype == QSV_C128 ? static_cast<const void*>(one) : onef,
-                                   h->amp_bytes(), cudaMemcpyHostToDevice, h->stream), "init");
+        if (h->dtype == QSV_C128) set_first<double>(S128(h), h->stream);
+        else set_first<float>(S64(h), h->stream);
+    });
+}
+
+int qsv_reset(void* hp) {
+    if (int rc = qsv_reset_async(hp)) return rc;
+    return guarded([&] {
+        Handle* h = H_(hp);
         check_cuda(cudaStreamSynchronize(h->stream), "init");
     });
 }

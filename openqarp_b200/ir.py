@@ -26,6 +26,12 @@ import numpy as np
 
 from .errors import CapabilityError
 
+try:
+    from . import _packc
+except ImportError as e:
+    raise ImportError("openqarp_b200/_packc.so (the command packer) is missing or does not load: build it with "
+                      "`make -C openqarp_b200/csrc` (or __graft_entry__.build()).") from e
+
 
 class GateType(enum.IntEnum):
     X = 0
@@ -322,21 +328,6 @@ def _gate_code(g) -> int:
     return int(v)
 
 
-_FAST: dict = {}
-
-
-def _fast_struct(nq: int, nv: int) -> struct.Struct:
-    """Header + qubits (+ padding to 8 bytes) + params of a command without cbits, conditions
-    or a matrix, as one struct."""
-    key = (nq, nv)
-    st = _FAST.get(key)
-    if st is None:
-        pad = (8 - (8 + 4 * nq) % 8) % 8
-        st = struct.Struct(f"<HBBBBBB{nq}I{pad}x{nv}d")
-        _FAST[key] = st
-    return st
-
-
 def _cmd_fields(cmd):
     g = _gate_code(cmd.gate)
     qubits = [int(q) for q in cmd.qubits]
@@ -374,19 +365,17 @@ def pack(commands: Iterable, values: Optional[Mapping[str, float]] = None,
     dep_ptr = [0]
     dep_param: list[int] = []
     dep_alpha: list[float] = []
+    commands = commands if type(commands) is list else list(commands)
+    if values is not None and type(values) is not dict:
+        values = dict(values)
     n = 0
-    for cmd in commands:
-        # common case: a plain gate of this module's Command with numeric parameters
-        if (type(cmd) is Command and not cmd.cbits and not cmd.condition_bits and cmd.unitary is None
-                and all(type(p) is float or type(p) is int for p in cmd.params)):
-            qs, ps = cmd.qubits, cmd.params
-            if len(qs) > 255 or len(ps) > 255:
-                raise ValueError("command too wide to pack")
-            out += _fast_struct(len(qs), len(ps)).pack(int(cmd.gate), len(qs), len(ps), 0, 0, 0, 0, *qs, *ps)
-            if index is not None:
-                dep_ptr.append(len(dep_param))
-            n += 1
-            continue
+    while True:
+        # plain gates, affine parameters and matrices of this module's types are packed natively, up
+        # to the next command of another form
+        n = _packc.pack(commands, n, out, Command, Param, values, index, dep_ptr, dep_param, dep_alpha)
+        if n >= len(commands):
+            break
+        cmd = commands[n]
         if isinstance(cmd, (PermutationRecord, ControlledUnitaryRecord)):
             _pack_record(out, cmd)
             if index is not None:
@@ -510,6 +499,32 @@ def measurements_are_terminal(commands: Sequence) -> bool:
 
 
 _RESET, _MEASURE, _BRANCH_BEGIN = int(GateType.Reset), int(GateType.Measure), int(GateType.BranchBegin)
+
+
+def any_needs_trajectory(commands) -> bool:
+    """Whether any command forces per-shot trajectories."""
+    got = _packc.needs_trajectory(commands, Command) if type(commands) is list else None
+    return any(needs_trajectory(c) for c in commands) if got is None else got
+
+
+def record_widths(buf: bytes) -> list:
+    """Qubit counts of a packed stream's records, barriers, measurements, global phases and records
+    without qubits left out."""
+    skip = (GateType.Barrier, GateType.Measure, GateType.GPhase)
+    out = []
+    off, end = 0, len(buf)
+    while off < end:
+        g, nq, npar, ncb, _flags, ncond, _ = _HDR.unpack_from(buf, off)
+        if nq and g not in skip:
+            out.append(nq)
+        off = ((off + _HDR.size + 4 * (nq + ncb + 2 * ncond) + 7) & ~7) + 8 * npar
+        if g == PERMUTATION_CODE:
+            off += 8 << nq
+        elif g == CONTROLLED_UNITARY_CODE:
+            off += 16 << (2 * nq - 2)
+        elif g == GateType.Custom:
+            off += 16 << (2 * nq)
+    return out
 
 
 def needs_trajectory(cmd) -> bool:

@@ -18,8 +18,8 @@ import numpy as np
 from . import _lib
 from ._lib import check, dptr, i32ptr, lib, u64ptr, u8ptr
 from .errors import CapabilityError
-from .ir import (PackedStream, cbit_register_width, measurements_are_terminal, needs_trajectory,
-                 pack)
+from .ir import (PackedStream, any_needs_trajectory, cbit_register_width, measurements_are_terminal, pack,
+                 record_widths)
 from .noise import as_noise_model
 from .observable import PauliMasks, to_masks
 from .program import GatesKernel, as_program
@@ -72,6 +72,11 @@ class Register:
     # state ---------------------------------------------------------------------------
     def reset(self):
         check(lib.qsv_reset(self.handle))
+
+    def _reset_async(self):
+        """reset() in stream order, without waiting: for callers that go on working on the register's
+        stream."""
+        check(lib.qsv_reset_async(self.handle))
 
     def set_state(self, amps, validate: bool = True):
         a = np.ascontiguousarray(np.asarray(amps, dtype=np.complex128).reshape(-1))
@@ -397,30 +402,24 @@ class B200Simulator:
 
     def _plan_widths(self, buf: bytes, n_qubits: int) -> list:
         """Widths of the fused commands the register's knobs apply to ``buf``."""
-        from .ir import GateType, unpack
         k = (self.last_plan or {}).get("fusion_k", self._fusion_max)
         size = ctypes.c_size_t()
-        check(lib.qsv_fuse_plan(u8ptr(buf), len(buf), n_qubits, int(k), self._fusion_min, None, 0,
-                                ctypes.byref(size)))
-        raw = ctypes.create_string_buffer(max(size.value, 1))
-        check(lib.qsv_fuse_plan(u8ptr(buf), len(buf), n_qubits, int(k), self._fusion_min, raw, size,
-                                ctypes.byref(size)))
-        skip = (GateType.Barrier, GateType.Measure, GateType.GPhase)
-        out = []
-        for c in unpack(raw.raw[:size.value]):
-            qs = getattr(c, "qubits", ()) or getattr(c, "targets", ())
-            if getattr(c, "gate", None) in skip or not qs:
-                continue
-            out.append(len(qs) + (1 if hasattr(c, "control") else 0))
-        return out
+        cap = 2 * len(buf) + 4096        # fused blocks of a few qubits rarely outgrow their gates' records
+        while True:
+            raw = ctypes.create_string_buffer(cap)
+            check(lib.qsv_fuse_plan(u8ptr(buf), len(buf), n_qubits, int(k), self._fusion_min, raw, cap,
+                                    ctypes.byref(size)))
+            if size.value <= cap:
+                return record_widths(raw.raw[:size.value])
+            cap = size.value
 
     def _state_report(self, reg: Register, buf: bytes, n_qubits: int):
         """Norm check, FP64 renormalisation and the a-priori bound after a complex64 apply."""
         from .precision import Complex64Report, plan_bound
+        widths = self._plan_widths(buf, n_qubits)      # host work, while the circuit runs
         n2 = reg.norm2()
         if self.renormalize and n2 > 0:
             reg.scale(1.0 / np.sqrt(n2))
-        widths = self._plan_widths(buf, n_qubits)
         stream_tensor = (self.last_plan or {}).get("executor", 0) == 0
         return Complex64Report(mode=self.error_report or "bound", norm2=n2, norm_drift=abs(n2 - 1.0),
                                commands=len(widths),
@@ -476,7 +475,7 @@ class B200Simulator:
             def seed():
                 reg.set_state(a, validate=True)
         else:
-            seed = reg.reset
+            seed = reg._reset_async
         buf = pack(commands, values).buf
         self._plan_for(reg, commands, buf, seed)
         seed()
@@ -513,7 +512,7 @@ class B200Simulator:
         extension) receives the amplitudes instead of a new array: a contiguous complex128
         array of length 2^n, e.g. in pinned host memory for a faster copy."""
         commands = list(commands)
-        if any(needs_trajectory(c) for c in commands):
+        if any_needs_trajectory(commands):
             raise RuntimeError(
                 "QarpSimulator::statevector: circuit contains mid-circuit measurement, Reset, or "
                 "classical condition — statevector is not deterministic. Use run() for trajectory "
@@ -605,7 +604,7 @@ class B200Simulator:
         prog = as_program(program)
         _check_program_width(prog, n_qubits, "program_statevector")
         for k in prog.kernels():
-            if isinstance(k, GatesKernel) and any(needs_trajectory(c) for c in k.commands):
+            if isinstance(k, GatesKernel) and any_needs_trajectory(list(k.commands)):
                 raise RuntimeError(
                     "QarpSimulator::program_statevector: program contains mid-circuit "
                     "measurement, Reset, or classical condition — statevector is not "
@@ -629,7 +628,7 @@ class B200Simulator:
                 continue
             if i + 1 == len(kernels):
                 last = list(k.commands)
-            elif any(needs_trajectory(c) for c in k.commands):
+            elif any_needs_trajectory(list(k.commands)):
                 raise ValueError("QarpSimulator::program_run: a measurement or classical condition "
                                  "outside the program's last gates kernel")
         if last is not None and not measurements_are_terminal(last):
@@ -672,7 +671,7 @@ class B200Simulator:
         """Re <psi|H|psi> with psi = circuit(initial or |0...0>), computed on the device
         (QarpSimulator::expectation, qarp_simulator.cpp:945-952)."""
         commands = list(commands)
-        if any(needs_trajectory(c) for c in commands):
+        if any_needs_trajectory(commands):
             raise RuntimeError("QarpSimulator::statevector: circuit contains mid-circuit measurement, "
                                "Reset, or classical condition — statevector is not deterministic.")
         self._refuse_noise(_NOISY_STATEVECTOR)
@@ -743,7 +742,7 @@ class B200Simulator:
     def energy_and_gradient(self, commands, n_qubits, observable, params, param_order, *,
                             initial_state=None):
         commands = list(commands)
-        if any(needs_trajectory(c) for c in commands):
+        if any_needs_trajectory(commands):
             raise RuntimeError("QarpSimulator::run_gradient: trajectory commands (Measure / Reset / "
                                "classical condition) are not differentiable.")
         masks = to_masks(observable, n_qubits, where="run_gradient")
@@ -759,10 +758,10 @@ class B200Simulator:
         energy, grad = reg.adjoint(stream, len(param_order), masks)
         if self._c64:
             from .precision import Complex64Report, h_norm1, plan_bound
-            d = plan_bound(self._plan_widths(stream.buf, n_qubits), 5)
+            widths = self._plan_widths(stream.buf, n_qubits)
+            d = plan_bound(widths, 5)
             h1 = h_norm1(masks)
-            rep = Complex64Report(mode=self.error_report or "bound",
-                                  commands=len(self._plan_widths(stream.buf, n_qubits)),
+            rep = Complex64Report(mode=self.error_report or "bound", commands=len(widths),
                                   l2_bound=d, value_bound=2 * h1 * d + h1 * d * d)
             sh = self._shadow_sim()
             if sh is not None:
@@ -777,7 +776,7 @@ class B200Simulator:
     def run_gradient_phi(self, commands, n_qubits: int, phi, params, param_order, *,
                          initial_state=None) -> list:
         commands = list(commands)
-        if any(needs_trajectory(c) for c in commands):
+        if any_needs_trajectory(commands):
             raise RuntimeError("QarpSimulator::run_gradient: trajectory commands (Measure / Reset / "
                                "classical condition) are not differentiable.")
         stream = pack(commands, dict(params), list(param_order))
@@ -793,12 +792,12 @@ class B200Simulator:
                                  f"2^n_qubits = {1 << n_qubits}")
             reg.set_state(a, validate=True)
         else:
-            reg.reset()
+            reg._reset_async()
 
     def unitary_matrix(self, commands, n_qubits: int) -> np.ndarray:
         """Full 2^n x 2^n unitary, column by column, unfused (qarp_simulator.cpp:1271-1304)."""
         commands = list(commands)
-        if any(needs_trajectory(c) for c in commands):
+        if any_needs_trajectory(commands):
             raise RuntimeError("QarpSimulator::unitary_matrix: circuit contains mid-circuit "
                                "measurement, Reset, or classical condition — output is not unitary.")
         self._refuse_noise("QarpSimulator::unitary_matrix: noise model is active — noisy evolution is "
