@@ -169,7 +169,9 @@ QSV_API int qsv_set_checkpoint_interval(void* h, int k);
 
 /* Register <- |0...0>. */
 QSV_API int qsv_reset(void* h);
-/* The same in stream order, without waiting for it. */
+/* The same in stream order, without waiting for it.  Until the next call on this handle nothing else may
+ * write to the register: if that call is qsv_apply or qsv_adjoint, its compiled tile passes leave out
+ * the tiles that a circuit from |0...0> has not reached yet. */
 QSV_API int qsv_reset_async(void* h);
 /* Register <- caller amplitudes (interleaved c128, len = 2^n).  validate != 0 checks
  * the norm within 1e-10 exactly as validate_initial_state (qarp_simulator.cpp:731-746). */

@@ -625,8 +625,9 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_adj_tile(vec2_t<T>* __restri
 
 // Encode the passes for the device and launch them in order on `st`.
 template <typename T>
-void run_tiled(const std::vector<TilePass>& passes, vec2_t<T>* s, int n, cudaStream_t st, Workspace& ws,
-               const std::function<void(const Op&)>& stream_op, bool register_tiles, bool jit) {
+double run_tiled(const std::vector<TilePass>& passes, vec2_t<T>* s, int n, cudaStream_t st, Workspace& ws,
+                 const std::function<void(const Op&)>& stream_op, bool register_tiles, bool jit, uint64_t support) {
+    double processed = 0;
     // compiled passes first (complex128), then the register-tile interpreter, then shared-memory ops
     JitPlan jp;
     if (jit) {
@@ -764,8 +765,11 @@ void run_tiled(const std::vector<TilePass>& passes, vec2_t<T>* s, int n, cudaStr
     int pi = 0;
     for (size_t i = 0; i < passes.size(); ++i) {
         const TilePass& p = passes[i];
+        const double whole = static_cast<double>(1ull << n);
         if (p.tile_qubits.empty()) {
             for (const Op& o : p.ops) stream_op(o);
+            support = ~0ull;
+            processed += whole;
             continue;
         }
         const uint64_t pass_bytes = 2ull * (1ull << n) * sizeof(vec2_t<T>);
@@ -773,12 +777,21 @@ void run_tiled(const std::vector<TilePass>& passes, vec2_t<T>* s, int n, cudaStr
         for (const Op& o : p.ops) pass_flops += op_flops_per_amp(o);
         pass_flops *= static_cast<double>(1ull << n);
         if (!jp.idx.empty() && jp.idx[i] >= 0) {
-            ws.timer.begin(st, "tile_jit", pass_bytes,
-                           jp.flops_per_amp[static_cast<size_t>(jp.idx[i])] * static_cast<double>(1ull << n));
-            jit_launch(jp, static_cast<int>(i), s, n, st);
+            uint64_t tile = 0, tmask = 0;
+            for (uint32_t q : p.tile_qubits) tile |= 1ull << q;
+            for (int q = 0, j = 0; q < n; ++q)
+                if (!((tile >> q) & 1)) tmask |= ((support >> q) & 1) << j++;
+            const double amps = static_cast<double>(1ull << (p.tile_qubits.size() + __builtin_popcountll(tmask)));
+            ws.timer.begin(st, "tile_jit", static_cast<uint64_t>(2 * amps * sizeof(vec2_t<T>)),
+                           jp.flops_per_amp[static_cast<size_t>(jp.idx[i])] * amps);
+            jit_launch(jp, static_cast<int>(i), s, n, tmask, st);
             ws.timer.end(st);
+            for (const Op& o : p.ops) support |= op_mixing_mask(o);
+            processed += amps;
             continue;
         }
+        support = ~0ull;
+        processed += whole;
         if (rt_idx[i] >= 0) {
             ws.timer.begin(st, "tile_rt", pass_bytes, pass_flops);
             launch_rt<T>(rt, rt_idx[i], s, n, st);
@@ -799,6 +812,7 @@ void run_tiled(const std::vector<TilePass>& passes, vec2_t<T>* s, int n, cudaStr
         ++pi;
     }
     // `host` is pageable: cudaMemcpyAsync returned only after staging it, so it may go now
+    return processed;
 }
 
 unsigned adjoint_tile_grid(int n, int m) {
@@ -1013,9 +1027,9 @@ template void run_adjoint_tiled<float>(const std::vector<Op>&, float2*, float2*,
                                        cudaStream_t, Workspace&, const std::function<void(const Op&)>&, uint64_t*,
                                        std::vector<int>*);
 
-template void run_tiled<double>(const std::vector<TilePass>&, double2*, int, cudaStream_t, Workspace&,
-                                const std::function<void(const Op&)>&, bool, bool);
-template void run_tiled<float>(const std::vector<TilePass>&, float2*, int, cudaStream_t, Workspace&,
-                               const std::function<void(const Op&)>&, bool, bool);
+template double run_tiled<double>(const std::vector<TilePass>&, double2*, int, cudaStream_t, Workspace&,
+                                  const std::function<void(const Op&)>&, bool, bool, uint64_t);
+template double run_tiled<float>(const std::vector<TilePass>&, float2*, int, cudaStream_t, Workspace&,
+                                 const std::function<void(const Op&)>&, bool, bool, uint64_t);
 
 }  // namespace qsv

@@ -1085,6 +1085,13 @@ __device__ __forceinline__ double flip(double a, int m) {
     return __hiloint2double(__double2hiint(a) ^ m, __double2loint(a));
 }
 __device__ __forceinline__ float flip(float a, int m) { return __int_as_float(__float_as_int(a) ^ m); }
+// the bits of i placed at the set bits of m, lowest first
+__device__ __forceinline__ u64 spread(u64 i, u64 m) {
+    u64 r = 0;
+    for (; i && m; i >>= 1, m &= m - 1)
+        if (i & 1) r |= m & (0 - m);
+    return r;
+}
 __device__ __forceinline__ void cp16(void* dst, const void* src) {
     const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(src) : "memory");
@@ -1301,7 +1308,7 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
     }
     s << "struct __align__(8) C" << idx << " { R c[" << nc << "]; };\n"
       << "extern \"C\" __global__ void __launch_bounds__(" << kJitThreads << ", " << (pair ? 1 : jit_ctas(f32))
-      << ") qsv_jit_" << idx << "(R2* __restrict__ s, u64 n_tiles, u64 turned, "
+      << ") qsv_jit_" << idx << "(R2* __restrict__ s, u64 n_tiles, u64 tmask, u64 tstep, u64 turned, "
       << (pair ? "R2* __restrict__ s2, double2* __restrict__ partials, " : "") << "const __grid_constant__ C" << idx << " P"
       << (kJitDebug ? ", unsigned long long* __restrict__ dbg" : "") << ") {\n"
       << "  extern __shared__ __align__(16) unsigned char smem[];\n"
@@ -1315,10 +1322,12 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
       << "  const u64 gtid = " << gtid << ";\n"
       << "  const unsigned stid = swz(tid);\n"
       << "  const u64 gfin = " << gfin << ";\n"
-      << "  u64 t = blockIdx.x;\n"
-      << "  if (t < n_tiles) {\n    const u64 b0 = " << deposit("t") << ";\n" << issue("b0") << "  }\n"
+      // the i-th tile is the i-th subset of tmask; tstep = spread(gridDim.x, tmask), added with the
+      // carries running through the other bits
+      << "  u64 i = blockIdx.x, t = spread(i, tmask);\n"
+      << "  if (i < n_tiles) {\n    const u64 b0 = " << deposit("t") << ";\n" << issue("b0") << "  }\n"
       << "  asm volatile(\"cp.async.commit_group;\\n\" ::: \"memory\");\n"
-      << "  for (; t < n_tiles; t += gridDim.x) {\n"
+      << "  for (; i < n_tiles; i += gridDim.x, t = ((t | ~tmask) + tstep) & tmask) {\n"
       << "  const u64 base = " << deposit("t") << ";\n"
       << "  asm volatile(\"cp.async.wait_group 0;\\n\" ::: \"memory\");\n"
       << "  __syncthreads();\n"
@@ -1343,7 +1352,7 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
     s << "  }\n  __syncthreads();\n"
       << steps
       << "  __syncthreads();\n"
-      << "  if (t + gridDim.x < n_tiles) {\n    const u64 tn = t + gridDim.x;\n    const u64 b1 = " << deposit("tn")
+      << "  if (i + gridDim.x < n_tiles) {\n    const u64 tn = ((t | ~tmask) + tstep) & tmask;\n    const u64 b1 = " << deposit("tn")
       << ";\n" << issue("b1") << "  }\n"
       << "  asm volatile(\"cp.async.commit_group;\\n\" ::: \"memory\");\n";
     s << "  const u64 to = (base | gfin) ^ turned;\n";
@@ -1672,20 +1681,25 @@ JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int devic
 }
 
 namespace {
-void launch_pass(const JitPlan& plan, int pass, void* s, void* s2, double2* partials, int n, cudaStream_t st) {
+void launch_pass(const JitPlan& plan, int pass, void* s, void* s2, double2* partials, int n, unsigned long long tmask,
+                 cudaStream_t st) {
     const int k = plan.idx.at(pass);
     if (k < 0) throw std::logic_error("JIT tiles: pass was not compiled");
     int sms = 0, device = 0;
     check_cuda(cudaGetDevice(&device), "device");
     check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "sm count");
-    unsigned long long n_tiles = 1ull << (n - kRtQubits);
+    tmask &= (1ull << (n - kRtQubits)) - 1;
+    unsigned long long n_tiles = 1ull << __builtin_popcountll(tmask);
     const int ctas = plan.pair ? 1 : jit_ctas(plan.f32);
     const unsigned grid = static_cast<unsigned>(
         std::min<unsigned long long>(n_tiles, static_cast<unsigned long long>(ctas) * sms));
     const std::vector<uint8_t>& c = plan.coef[static_cast<size_t>(k)];
     unsigned long long turned = plan.turned[static_cast<size_t>(k)];
+    unsigned long long tstep = 0;      // spread(grid, tmask)
+    for (unsigned long long i = grid, m = tmask; i && m; i >>= 1, m &= m - 1)
+        if (i & 1) tstep |= m & (0 - m);
     double2* part = partials ? partials + static_cast<size_t>(plan.acc0[static_cast<size_t>(k)]) * grid : nullptr;
-    std::vector<void*> args{&s, &n_tiles, &turned};
+    std::vector<void*> args{&s, &n_tiles, &tmask, &tstep, &turned};
     if (plan.pair) args.insert(args.end(), {static_cast<void*>(&s2), static_cast<void*>(&part)});
     args.push_back(const_cast<uint8_t*>(c.data()));
 #ifdef QSV_DEBUG_BOUNDS
@@ -1699,12 +1713,12 @@ void launch_pass(const JitPlan& plan, int pass, void* s, void* s2, double2* part
 }
 }  // namespace
 
-void jit_launch(const JitPlan& plan, int pass, void* s, int n, cudaStream_t st) {
-    launch_pass(plan, pass, s, nullptr, nullptr, n, st);
+void jit_launch(const JitPlan& plan, int pass, void* s, int n, uint64_t tmask, cudaStream_t st) {
+    launch_pass(plan, pass, s, nullptr, nullptr, n, tmask, st);
 }
 
 void jit_launch_pair(const JitPlan& plan, int pass, void* psi, void* phi, double2* partials, int n, cudaStream_t st) {
-    launch_pass(plan, pass, psi, phi, partials, n, st);
+    launch_pass(plan, pass, psi, phi, partials, n, ~0ull, st);
 }
 
 bool run_adjoint_compiled(const std::vector<Op>& ops, double2* psi, double2* phi, int n, double2* partials, unsigned nb,

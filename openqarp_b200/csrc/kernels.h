@@ -151,10 +151,14 @@ bool apply_ops_small(const std::vector<Op>& ops, vec2_t<T>* s, int n, cudaStream
 // ---------------------------------------------------------------- tiled executor (kern_tile.cu)
 // Launch the planned passes; one-op stream passes (empty tile_qubits) go to `stream_op`.
 // With register_tiles, passes plan_rt accepts run on the register-tile kernel.
-// With jit (complex128), passes the JIT generator handles run as compiled straight-line kernels.
+// With jit, passes the JIT generator handles run as compiled straight-line kernels.
+// `support`: qubits whose bit is 1 in some nonzero amplitude (~0: unknown).  Tiles whose other qubits are
+// not all inside it hold zeros and stay so: the compiled passes leave them out (a circuit from |0...0>
+// reaches all of 28 qubits only in its fourth pass).  Returns the amplitudes the passes processed.
 template <typename T>
-void run_tiled(const std::vector<TilePass>& passes, vec2_t<T>* s, int n, cudaStream_t st, Workspace& ws,
-               const std::function<void(const Op&)>& stream_op, bool register_tiles, bool jit = false);
+double run_tiled(const std::vector<TilePass>& passes, vec2_t<T>* s, int n, cudaStream_t st, Workspace& ws,
+                 const std::function<void(const Op&)>& stream_op, bool register_tiles, bool jit = false,
+                 uint64_t support = ~0ull);
 
 // ---------------------------------------------------------------- JIT register tiles (kern_tile_jit.cu)
 // The register-tile passes of a stream compiled to straight-line kernels.
@@ -179,7 +183,9 @@ struct JitPlan {
 // `pair`: passes of the adjoint's reverse sweep over psi and phi (complex128); then every tile pass
 // compiles, or the plan comes back empty (idx empty).
 JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int device, bool f32, bool pair = false);
-void jit_launch(const JitPlan& plan, int pass, void* s, int n, cudaStream_t st);
+// tmask: which tile-number bits (the qubits outside the tile, ascending) run through both values; the
+// others stay 0 (~0: the whole register)
+void jit_launch(const JitPlan& plan, int pass, void* s, int n, uint64_t tmask, cudaStream_t st);
 // accumulator a's partial of block b goes to partials[a * grid + b].x, grid = adjoint_tile_grid(n, kRtQubits)
 void jit_launch_pair(const JitPlan& plan, int pass, void* psi, void* phi, double2* partials, int n, cudaStream_t st);
 // host-only helpers for plan inspection and tests (no device work)

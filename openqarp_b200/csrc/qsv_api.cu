@@ -161,6 +161,7 @@ struct Handle {
     std::vector<void*> ckpt;      // adjoint: |psi> checkpoint buffers kept between calls
     size_t ckpt_bytes = 0;        // size of each
     int checkpoint_interval = -1; // adjoint: commands between psi checkpoints (-1 auto, 0 none)
+    bool zero_state = false;      // |0...0> since qsv_reset_async, nothing else done with the register
     uint64_t traj_batch = 0;      // trajectories: shots per device batch (0: memory-bound default)
     std::vector<NoiseSpec> noise; // trajectories: channel per gate type (empty: noiseless)
     uint64_t dim() const { return 1ull << n; }
@@ -209,9 +210,12 @@ int guarded(F&& f) {
     }
 }
 
-Handle* H_(void* h) {
+// The handle of an entry point.  `keep`: the call neither writes to the register nor lets the caller do
+// so; every other one ends what qsv_reset_async promised about it.
+Handle* H_(void* h, bool keep = false) {
     if (!h) throw std::invalid_argument("null handle");
     Handle* p = static_cast<Handle*>(h);
+    if (!keep) p->zero_state = false;
     check_cuda(cudaSetDevice(p->device), "cudaSetDevice");
     return p;
 }
@@ -277,6 +281,8 @@ void apply_stream(Handle* h, const uint8_t* buf, size_t nbytes, bool fuse) {
 }
 
 void apply_cmds(Handle* h, std::vector<Cmd> cmds, bool fuse) {
+    const uint64_t support = h->zero_state ? 0 : ~0ull;
+    h->zero_state = false;
     check_stream(cmds);
     if (fuse) cmds = fuse_for_dispatch(cmds, h->n, h->fusion_max, h->fusion_min);
     std::vector<Op> ops;
@@ -295,16 +301,20 @@ void apply_cmds(Handle* h, std::vector<Cmd> cmds, bool fuse) {
         auto stream_op = [h](const Op& o) { launch(h, o, h->state); };
         const bool rt = h->executor == 1 || h->executor == 3;
         const bool jit = h->executor == 3;
-        if (h->dtype == QSV_C128) run_tiled<double>(passes, S128(h), h->n, h->stream, h->ws, stream_op, rt, jit);
-        else run_tiled<float>(passes, S64(h), h->n, h->stream, h->ws, stream_op, rt, jit);
+        double amps = h->dtype == QSV_C128
+                          ? run_tiled<double>(passes, S128(h), h->n, h->stream, h->ws, stream_op, rt, jit, support)
+                          : run_tiled<float>(passes, S64(h), h->n, h->stream, h->ws, stream_op, rt, jit, support);
         for (const TilePass& p : passes) {
-            if (p.tile_qubits.empty()) continue;   // counted by launch()
+            if (p.tile_qubits.empty()) {   // counted by launch()
+                amps -= static_cast<double>(h->dim());
+                continue;
+            }
             h->stats.launches++;
             h->stats.passes++;
-            h->stats.hbm_bytes += 2ull * h->dim() * h->amp_bytes();
             for (const Op& o : p.ops)
                 if (o.kind == OP_DENSE && o.k >= 2) h->stats.fused_blocks++;
         }
+        h->stats.hbm_bytes += static_cast<uint64_t>(2.0 * amps) * h->amp_bytes();
     } else {
         h->ws.timer.begin(h->stream, "fs_apply", 2ull * h->dim() * h->amp_bytes());
         const bool small = h->dtype == QSV_C128 ? apply_ops_small<double>(ops, S128(h), h->n, h->stream, h->ws)
@@ -494,7 +504,7 @@ int qsv_destroy(void* hp) {
 
 int qsv_set_fusion(void* hp, int max_q, int min_q) {
     return guarded([&] {
-        Handle* h = H_(hp);
+        Handle* h = H_(hp, true);
         if (max_q < 0 || max_q > QSV_MAX_BLOCK_QUBITS)
             throw std::invalid_argument("QarpSimulator::set_fusion_max_qubits: " + std::to_string(max_q) +
                                         " exceeds the maximum block width " +
@@ -507,7 +517,7 @@ int qsv_set_fusion(void* hp, int max_q, int min_q) {
 
 int qsv_set_executor(void* hp, int mode) {
     return guarded([&] {
-        Handle* h = H_(hp);
+        Handle* h = H_(hp, true);
         if (mode < -1 || mode > 3) throw std::invalid_argument("executor mode must be -1, 0, 1, 2 or 3");
         h->executor = mode;
     });
@@ -515,7 +525,7 @@ int qsv_set_executor(void* hp, int mode) {
 
 int qsv_set_checkpoint_interval(void* hp, int k) {
     return guarded([&] {
-        Handle* h = H_(hp);
+        Handle* h = H_(hp, true);
         if (k < -1) throw std::invalid_argument("checkpoint interval must be -1 (default), 0 (none) or > 0");
         h->checkpoint_interval = k;
     });
@@ -557,7 +567,7 @@ int qsv_set_trajectory_batch(void* hp, uint64_t max_shots) {
 
 int qsv_set_tile_qubits(void* hp, int m) {
     return guarded([&] {
-        Handle* h = H_(hp);
+        Handle* h = H_(hp, true);
         if (m != 0 && (m < kTileMinQubits || m > kTileMaxQubits))
             throw std::invalid_argument("tile qubits must be 0 (default) or in [" + std::to_string(kTileMinQubits) +
                                         ", " + std::to_string(kTileMaxQubits) + "]");
@@ -574,13 +584,14 @@ int qsv_reset_async(void* hp) {
         check_cuda(cudaMemsetAsync(h->state, 0, h->dim() * h->amp_bytes(), h->stream), "memset");
         if (h->dtype == QSV_C128) set_first<double>(S128(h), h->stream);
         else set_first<float>(S64(h), h->stream);
+        h->zero_state = true;
     });
 }
 
 int qsv_reset(void* hp) {
     if (int rc = qsv_reset_async(hp)) return rc;
     return guarded([&] {
-        Handle* h = H_(hp);
+        Handle* h = H_(hp);    // the caller may write through the device pointer before it applies
         check_cuda(cudaStreamSynchronize(h->stream), "init");
     });
 }
@@ -766,7 +777,7 @@ int qsv_debug_bounds_selftest(int device, int32_t* caught_in, int32_t* caught_ou
 int qsv_apply(void* hp, const uint8_t* cmds, size_t nbytes) {
     Range range("qsv_apply");
     return guarded([&] {
-        Handle* h = H_(hp);
+        Handle* h = H_(hp, true);
         if (!cmds && nbytes) throw std::invalid_argument("null command buffer");
         apply_stream(h, cmds, nbytes, true);
     });
@@ -1046,7 +1057,7 @@ int qsv_cbatch_destroy(void* b) {
 
 int qsv_synchronize(void* hp) {
     return guarded([&] {
-        Handle* h = H_(hp);
+        Handle* h = H_(hp, true);
         check_cuda(cudaStreamSynchronize(h->stream), "synchronize");
     });
 }
@@ -1067,7 +1078,7 @@ int qsv_device_info(int device, char* name, size_t cap, int* cc_major, int* cc_m
 
 int qsv_set_timing(void* hp, int on) {
     return guarded([&] {
-        Handle* h = H_(hp);
+        Handle* h = H_(hp, true);
         h->ws.timer.enable(on != 0);
     });
 }
@@ -1386,7 +1397,7 @@ int qsv_adjoint(void* hp, const uint8_t* cmds, size_t nbytes, const int32_t* dep
                 const uint64_t* zm, const double* coeff, size_t nt, double* grad, double* energy) {
     Range range("qsv_adjoint");
     return guarded([&] {
-        Handle* h = H_(hp);
+        Handle* h = H_(hp, true);
         if (n_params < 0 || (n_params > 0 && !grad)) throw std::invalid_argument("bad gradient output");
         const std::vector<Cmd> cs = checked_adjoint_stream(cmds, nbytes, dep_ptr, dep_param, n_params, h->n);
         const PauliTerms t = terms_of(h, xm, zm, coeff, nt);
