@@ -67,7 +67,7 @@ struct TrPlan {
 TrPlan build_plan(const std::vector<Cmd>& suffix, int n, int n_cbits, int fusion_max, int fusion_min,
                   const std::vector<NoiseSpec>* noise);
 
-// Whole shots in one CTA's shared memory, for registers of 4 to 64 KiB (kern_traj_fused.cu).
+// Whole shots in one CTA's shared memory, for registers of up to 64 KiB (kern_traj_fused.cu).
 // Returns false, having done nothing, when the register is too wide or the plan holds a step the
 // kernel does not run (a permutation, a dense block wider than four qubits).
 template <typename T>

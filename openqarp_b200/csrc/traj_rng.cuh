@@ -37,38 +37,44 @@ constexpr int kMtM = 397;
 struct MtView {
     uint32_t* w;          // word i at w[i * stride]
     uint64_t stride;
-    uint32_t* idx;        // next word to temper (kMtN: twist first)
+    uint32_t* idx;        // the next word: [0, n) in the first generation, [n, 2n) in later ones
 
     QSV_HD uint32_t& at(int i) const { return w[static_cast<uint64_t>(i) * stride]; }
 
+    // The first twisted word needs words 0, 1 and m: the seeding chain stops at m, and next() takes
+    // it one word further per draw.  Seeding is a serial chain (624 steps, then as many of the
+    // twist, before a shot's first draw) and a shot usually draws a few dozen words.
     QSV_HD void seed(uint32_t s) const {
         uint32_t x = s;
         at(0) = x;
-        for (int i = 1; i < kMtN; ++i) {
+        for (int i = 1; i <= kMtM; ++i) {
             x = 1812433253u * (x ^ (x >> 30)) + static_cast<uint32_t>(i);
             at(i) = x;
         }
-        *idx = kMtN;
-    }
-
-    QSV_HD void twist() const {
-        constexpr uint32_t upper = 0x80000000u, lower = 0x7fffffffu, a = 0x9908b0dfu;
-        for (int k = 0; k < kMtN - kMtM; ++k) {
-            const uint32_t y = (at(k) & upper) | (at(k + 1) & lower);
-            at(k) = at(k + kMtM) ^ (y >> 1) ^ ((y & 1u) ? a : 0u);
-        }
-        for (int k = kMtN - kMtM; k < kMtN - 1; ++k) {
-            const uint32_t y = (at(k) & upper) | (at(k + 1) & lower);
-            at(k) = at(k + kMtM - kMtN) ^ (y >> 1) ^ ((y & 1u) ? a : 0u);
-        }
-        const uint32_t y = (at(kMtN - 1) & upper) | (at(0) & lower);
-        at(kMtN - 1) = at(kMtM - 1) ^ (y >> 1) ^ ((y & 1u) ? a : 0u);
         *idx = 0;
     }
 
+    // Word k of the next generation is formed when it is drawn, in place and in order: the words
+    // that the bulk twist reads there (k + 1 and k + m, or k + m - n of the new generation) are
+    // the ones that stand there now.
     QSV_HD uint32_t next() const {
-        if (*idx >= static_cast<uint32_t>(kMtN)) twist();
-        uint32_t y = at(static_cast<int>((*idx)++));
+        constexpr uint32_t upper = 0x80000000u, lower = 0x7fffffffu, a = 0x9908b0dfu;
+        const int i = static_cast<int>(*idx);
+        const int k = i < kMtN ? i : i - kMtN;
+        uint32_t far;
+        if (k < kMtN - kMtM) {
+            if (i < kMtN && k > 0) {   // not seeded yet
+                const uint32_t x = at(k + kMtM - 1);
+                at(k + kMtM) = 1812433253u * (x ^ (x >> 30)) + static_cast<uint32_t>(k + kMtM);
+            }
+            far = at(k + kMtM);
+        } else {
+            far = at(k + kMtM - kMtN);
+        }
+        const uint32_t m = (at(k) & upper) | (at(k + 1 < kMtN ? k + 1 : 0) & lower);
+        uint32_t y = far ^ (m >> 1) ^ ((m & 1u) ? a : 0u);
+        at(k) = y;
+        *idx = static_cast<uint32_t>(i + 1 < 2 * kMtN ? i + 1 : kMtN);
         y ^= y >> 11;
         y ^= (y << 7) & 0x9d2c5680u;
         y ^= (y << 15) & 0xefc60000u;
