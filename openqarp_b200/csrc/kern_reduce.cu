@@ -356,18 +356,53 @@ __global__ void __launch_bounds__(kRed, 2) k_apply_obs(const vec2_t<T>* __restri
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kRed) k_norm2(const vec2_t<T>* __restrict__ s, uint64_t dim, double2* __restrict__ partials) {
-    double2 acc = make_double2(0, 0);
-    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < dim; i += stride) {
-        const vec2_t<T> a = *QSV_DBG(s + i);
-        const double x = a.x, y = a.y;
-        acc.x = fma(x, x, acc.x);
-        acc.x = fma(y, y, acc.x);
+// |v|^2 of 16 bytes of a register (one complex128 amplitude or two complex64 ones), in FP64.
+// Widening a float by the conversion unit bounds a plain read of a complex64 register (5.2 TB/s at
+// 30 qubits), so it is widened by its bits: sign dropped, the rest shifted into place is |x| 2^-896
+// for every finite float, subnormal ones too, and a product with 2^896 is exact.  Infinities and
+// NaNs do not survive that; `top` keeps the largest magnitude's bits and overrides the sum.
+__device__ __forceinline__ double norm_of(double2 v, uint32_t&) { return fma(v.x, v.x, v.y * v.y); }
+__device__ __forceinline__ double magnitude(float x, uint32_t& top) {
+    const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
+    top = max(top, b);
+    return __hiloint2double(static_cast<int>(b >> 3), static_cast<int>(b << 29)) * 0x1p896;
+}
+__device__ __forceinline__ double norm_of(float2 v, uint32_t& top) {
+    const double a = magnitude(v.x, top), b = magnitude(v.y, top);
+    return fma(a, a, b * b);
+}
+__device__ __forceinline__ double norm_of(float4 v, uint32_t& top) {
+    return norm_of(make_float2(v.x, v.y), top) + norm_of(make_float2(v.z, v.w), top);
+}
+__device__ __forceinline__ float2 scaled(float2 v, double f) {
+    return make_float2(static_cast<float>(v.x * f), static_cast<float>(v.y * f));
+}
+__device__ __forceinline__ double2 scaled(double2 v, double f) { return make_double2(v.x * f, v.y * f); }
+__device__ __forceinline__ float4 scaled(float4 v, double f) {
+    return make_float4(static_cast<float>(v.x * f), static_cast<float>(v.y * f), static_cast<float>(v.z * f),
+                       static_cast<float>(v.w * f));
+}
+
+// Whole registers in 16-byte words, kWords in flight per thread; HBM bounds both.  Complex64, 30
+// qubits: norm 1.28 ms (6.9 TB/s; an 8-byte amplitude per load, widened by conversion, 1.83), scale
+// 2.47 ms (7.0 TB/s; 3.06).
+constexpr int kWords = 4;
+template <typename V>
+__global__ void __launch_bounds__(kRed) k_norm2(const V* __restrict__ s, uint64_t words, double2* __restrict__ partials) {
+    double acc[kWords] = {};
+    uint32_t top = 0;
+    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x * kWords;
+    for (uint64_t at = static_cast<uint64_t>(blockIdx.x) * blockDim.x * kWords + threadIdx.x; at < words; at += stride) {
+        V v[kWords] = {};
+#pragma unroll
+        for (int u = 0; u < kWords; ++u)
+            if (at + u * kRed < words) v[u] = *QSV_DBG(s + (at + u * kRed));
+#pragma unroll
+        for (int u = 0; u < kWords; ++u) acc[u] += norm_of(v[u], top);
     }
-    acc = block_sum(acc);
-    if (threadIdx.x == 0) *QSV_DBG(partials + blockIdx.x) = acc;
+    if (top >= 0x7f800000u) acc[0] = static_cast<double>(__uint_as_float(top));   // infinity or NaN
+    const double2 sum = block_sum(make_double2((acc[0] + acc[1]) + (acc[2] + acc[3]), 0.0));
+    if (threadIdx.x == 0) *QSV_DBG(partials + blockIdx.x) = sum;
 }
 
 template <typename TA, typename TB>
@@ -384,18 +419,18 @@ __global__ void __launch_bounds__(kRed) k_inner(const vec2_t<TA>* __restrict__ a
     if (threadIdx.x == 0) *QSV_DBG(partials + blockIdx.x) = v;
 }
 
-template <typename T>
 // the product is formed in FP64 and rounded once to the storage type: a renormalising factor
 // within 1e-8 of 1 would vanish if it were itself rounded to FP32 first
-__global__ void k_scale_real(vec2_t<T>* __restrict__ s, uint64_t dim, double f) {
-    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < dim; i += stride) {
-        vec2_t<T>* const si = QSV_DBG(s + i);
-        vec2_t<T> a = *si;
-        a.x = static_cast<T>(static_cast<double>(a.x) * f);
-        a.y = static_cast<T>(static_cast<double>(a.y) * f);
-        *si = a;
-    }
+template <typename V>
+__global__ void __launch_bounds__(kRed) k_scale_real(V* __restrict__ s, uint64_t words, double f) {
+    const uint64_t at = static_cast<uint64_t>(blockIdx.x) * kRed * kWords + threadIdx.x;
+    V v[kWords];
+#pragma unroll
+    for (int u = 0; u < kWords; ++u)
+        if (at + u * kRed < words) v[u] = *QSV_DBG(s + (at + u * kRed));
+#pragma unroll
+    for (int u = 0; u < kWords; ++u)
+        if (at + u * kRed < words) *QSV_DBG(s + (at + u * kRed)) = scaled(v[u], f);
 }
 
 template <typename T>
@@ -809,12 +844,29 @@ void apply_observable(const vec2_t<T>* psi, vec2_t<T>* out, int n, const PauliTe
     check_cuda(cudaGetLastError(), "observable launch");
 }
 
+// A whole register (on its allocation's boundary) as 16-byte words; the complex64 register of no
+// qubits has 8 bytes.
+template <typename F>
+void in_words(const double2* s, uint64_t dim, F f) { f(s, dim); }
+template <typename F>
+void in_words(double2* s, uint64_t dim, F f) { f(s, dim); }
+template <typename F>
+void in_words(const float2* s, uint64_t dim, F f) {
+    if (dim > 1) f(reinterpret_cast<const float4*>(s), dim / 2);
+    else f(s, dim);
+}
+template <typename F>
+void in_words(float2* s, uint64_t dim, F f) {
+    if (dim > 1) f(reinterpret_cast<float4*>(s), dim / 2);
+    else f(s, dim);
+}
+
 template <typename T>
 double norm2(const vec2_t<T>* s, int n, cudaStream_t st, Workspace& ws) {
     const uint64_t dim = 1ull << n;
     const unsigned nb = red_blocks(dim);
     double2* partials = static_cast<double2*>(ws.scratch((nb + 1) * sizeof(double2)));
-    k_norm2<T><<<nb, kRed, 0, st>>>(s, dim, partials);
+    in_words(s, dim, [&](auto* w, uint64_t words) { k_norm2<<<nb, kRed, 0, st>>>(w, words, partials); });
     check_cuda(cudaGetLastError(), "norm launch");
     double out[2];
     finish(partials, nb, st, ws, out);
@@ -835,7 +887,9 @@ void inner(const vec2_t<TA>* a, const vec2_t<TB>* b, int n, cudaStream_t st, Wor
 template <typename T>
 void scale_real(vec2_t<T>* s, int n, double f, cudaStream_t st) {
     const uint64_t dim = 1ull << n;
-    k_scale_real<T><<<grid_for(dim, 1, 1u << 20), kThreads, 0, st>>>(s, dim, f);
+    in_words(s, dim, [&](auto* w, uint64_t words) {
+        k_scale_real<<<static_cast<unsigned>((words + kRed * kWords - 1) / (kRed * kWords)), kRed, 0, st>>>(w, words, f);
+    });
     check_cuda(cudaGetLastError(), "scale launch");
 }
 
