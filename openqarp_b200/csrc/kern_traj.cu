@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kTrThreads) k_tr_apply_2x2(vec2_t<T>* __restri
 // chosen), and one pass applies the four operators to 16 amplitudes a thread, with the next four
 // qubits' sums on its way.  One qubit at a time read the register twice and wrote it once per
 // channel: 16 qubits, 1024 shots, 128 channels 60 ms; 17 ms so.  A pass takes 0.43 ms of 2 GiB moved
-// (0.70 where the four qubits include the lowest, whose 16-byte runs do not coalesce).  Measurements
+// (0.50 through shared memory where they are the lowest four).  Measurements
 // that follow one another are the same with projectors (16 final ones 6.2 -> 2.2 ms).
 constexpr int kKrausGroup = 4;
 constexpr int kKrausMinQubits = 12;        // a block's 4096 amplitudes belong to one shot
@@ -352,19 +352,38 @@ struct KrausPass {
 
 // Group index g names the amplitudes that differ in the MA applied qubits; bits 0..4 of g are the
 // lane, 5..7 the warp, then the thread's iterations and the block.
-template <typename T, int MA>
+// Where the block's amplitude i lies when qubits 0..3 are the ones applied (LOW): a thread's 16 are
+// consecutive then, and the place in a 128-byte row is XORed so that 8 (16) lanes cover all banks.
+template <typename T>
+__device__ __forceinline__ uint32_t low_place(uint32_t i) {
+    return i ^ ((i >> 4) & (sizeof(T) == 8 ? 7u : 15u));
+}
+
+// LOW: the applied qubits are 0..3, so a lane's amplitudes would be 256 bytes from the next lane's
+// (715 us at 26 qubits against 441 for higher qubits): the block's 4096 amplitudes go through shared
+// memory instead, read and written in order (498 us).
+template <typename T, int MA, bool LOW>
 __global__ void __launch_bounds__(kTrThreads, 2) k_tr_kraus_pass(vec2_t<T>* __restrict__ s, int n,
                                                              const __grid_constant__ KrausPass kp,
                                                              const int8_t* __restrict__ act,
                                                              const double* __restrict__ kmat,
                                                              double* __restrict__ sums) {
     constexpr int kIters = 16 >> MA;
+    static_assert(!LOW || MA == 4, "one round: a block's amplitudes are consecutive");
+    extern __shared__ __align__(16) unsigned char kraus_smem[];
+    vec2_t<T>* const tile = reinterpret_cast<vec2_t<T>*>(kraus_smem);   // LOW: 4096 amplitudes
     __shared__ double part[kIters * kTrThreads];
     const uint32_t tid = threadIdx.x;
     const uint64_t per_shot = 1ull << (n - kTrChunkLog);
     const uint64_t shot = blockIdx.x / per_shot, chunk = blockIdx.x % per_shot;
     vec2_t<T>* p = s + (shot << n);
     const int on = MA > 0 ? *QSV_DBG(act + shot) : 0;
+    vec2_t<T>* const mine = p + chunk * 4096u;   // LOW
+    if (LOW) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) tile[low_place<T>(j * kTrThreads + tid)] = *QSV_DBG(mine + (j * kTrThreads + tid));
+        __syncthreads();
+    }
     uint32_t sum_bits = 0;
     for (int k = 0; k < kp.n_sum; ++k) sum_bits |= 1u << kp.at[k];
 #pragma unroll 1
@@ -374,7 +393,7 @@ __global__ void __launch_bounds__(kTrThreads, 2) k_tr_kraus_pass(vec2_t<T>* __re
         double xr[1 << MA], xi[1 << MA];
 #pragma unroll
         for (int r = 0; r < (1 << MA); ++r) {
-            const vec2_t<T> v = *QSV_DBG(p + (base | kp.off[r]));
+            const vec2_t<T> v = LOW ? tile[low_place<T>(tid * 16u | kp.off[r])] : *QSV_DBG(p + (base | kp.off[r]));
             xr[r] = v.x;
             xi[r] = v.y;
         }
@@ -401,7 +420,11 @@ __global__ void __launch_bounds__(kTrThreads, 2) k_tr_kraus_pass(vec2_t<T>* __re
                 }
             }
 #pragma unroll
-            for (int r = 0; r < (1 << MA); ++r) *QSV_DBG(p + (base | kp.off[r])) = mk<T>(static_cast<T>(xr[r]), static_cast<T>(xi[r]));
+            for (int r = 0; r < (1 << MA); ++r) {
+                const vec2_t<T> v = mk<T>(static_cast<T>(xr[r]), static_cast<T>(xi[r]));
+                if (LOW) tile[low_place<T>(tid * 16u | kp.off[r])] = v;
+                else *QSV_DBG(p + (base | kp.off[r])) = v;
+            }
         }
         if (kp.n_sum) {
             double v = 0.0;
@@ -413,9 +436,13 @@ __global__ void __launch_bounds__(kTrThreads, 2) k_tr_kraus_pass(vec2_t<T>* __re
             part[it * kTrThreads + tid] = v;
         }
     }
-    if (!kp.n_sum) return;
+    if (!LOW && !kp.n_sum) return;
     __syncthreads();
-    if (tid >= (1u << kp.n_sum)) return;
+    if (LOW && on) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) *QSV_DBG(mine + (j * kTrThreads + tid)) = tile[low_place<T>(j * kTrThreads + tid)];
+    }
+    if (!kp.n_sum || tid >= (1u << kp.n_sum)) return;
     // sum `tid`: in every warp row whose bits match, the lane whose summed-over bits are 0
     uint64_t want = 0;
     for (int k = 0; k < kp.n_sum; ++k) want |= static_cast<uint64_t>((tid >> k) & 1u) << kp.at[k];
@@ -1242,11 +1269,21 @@ void run_trajectories(const std::vector<Cmd>& suffix, int n, int n_cbits, const 
                 }
                 const unsigned grid = static_cast<unsigned>(static_cast<uint64_t>(nb) << (n - kTrChunkLog));
                 switch (b - a) {
-                    case 0: k_tr_kraus_pass<T, 0><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
-                    case 1: k_tr_kraus_pass<T, 1><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
-                    case 2: k_tr_kraus_pass<T, 2><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
-                    case 3: k_tr_kraus_pass<T, 3><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
-                    default: k_tr_kraus_pass<T, 4><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                    case 0: k_tr_kraus_pass<T, 0, false><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                    case 1: k_tr_kraus_pass<T, 1, false><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                    case 2: k_tr_kraus_pass<T, 2, false><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                    case 3: k_tr_kraus_pass<T, 3, false><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho); break;
+                    default:
+                        if (applied == 15) {
+                            const size_t smem = 4096 * sizeof(vec2_t<T>);
+                            check_cuda(cudaFuncSetAttribute(k_tr_kraus_pass<T, 4, true>,
+                                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                            static_cast<int>(smem)), "Kraus pass smem");
+                            k_tr_kraus_pass<T, 4, true><<<grid, kTrThreads, smem, st>>>(s, n, kp, d_outcome, d_kmat, d_rho);
+                        } else {
+                            k_tr_kraus_pass<T, 4, false><<<grid, kTrThreads, 0, st>>>(s, n, kp, d_outcome, d_kmat, d_rho);
+                        }
+                        break;
                 }
                 n_launch++;
             };
