@@ -15,7 +15,7 @@
 // ~/.cache/openqarp_b200/jit).
 //
 // NVRTC and the CUDA driver API are opened with dlopen on first use, so the library loads
-// (and every other executor runs) where they are absent.  Complex128 only.
+// (and every other executor runs) where they are absent.
 #include <dlfcn.h>
 #include <sys/stat.h>
 #include <unistd.h>
