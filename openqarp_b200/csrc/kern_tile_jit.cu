@@ -1743,7 +1743,8 @@ void jit_launch_pair(const JitPlan& plan, int pass, void* psi, void* phi, double
 }
 
 bool run_adjoint_compiled(const std::vector<Op>& ops, double2* psi, double2* phi, int n, double2* partials, unsigned nb,
-                          cudaStream_t st, const std::function<void(const Op&)>& stream_op, uint64_t* launches, int* n_acc,
+                          cudaStream_t st, const std::function<void()>& settle,
+                          const std::function<void(const Op&)>& stream_op, uint64_t* launches, int* n_acc,
                           std::vector<JitPlan::Adj>* steps) {
     if (ops.empty()) return true;
     // a pass ends where its accumulators or its parameters would overflow (at most 32 doubles of phase
@@ -1784,6 +1785,7 @@ bool run_adjoint_compiled(const std::vector<Op>& ops, double2* psi, double2* phi
     check_cuda(cudaGetDevice(&device), "device");
     JitPlan plan = jit_prepare(ptrs, n, device, false, true);
     if (plan.idx.empty()) return false;
+    settle();
     for (size_t i = 0; i < passes.size(); ++i) {
         if (passes[i].tile_qubits.empty()) {
             for (const Op& o : passes[i].ops) stream_op(o);

@@ -205,15 +205,18 @@ void run_adjoint_tiled(const std::vector<Op>& ops, vec2_t<T>* psi, vec2_t<T>* ph
                        const std::function<void(const Op&)>& stream_op, uint64_t* launches,
                        std::vector<int>* slot_order = nullptr);
 // The same in compiled pair passes (complex128, kern_tile_jit.cu): accumulators from *n_acc on, partials
-// [accumulator][block] in .x, steps' weighted sums appended to `steps`.  False, having done nothing, when
-// a pass cannot be compiled.
+// [accumulator][block] in .x, steps' weighted sums appended to `steps`.  psi and phi have to be the true
+// states, no factor left out: `settle` is called once every pass is compiled, before the first runs.
+// False, having done nothing, when a pass cannot be compiled.
 bool run_adjoint_compiled(const std::vector<Op>& ops, double2* psi, double2* phi, int n, double2* partials, unsigned nb,
-                          cudaStream_t st, const std::function<void(const Op&)>& stream_op, uint64_t* launches, int* n_acc,
+                          cudaStream_t st, const std::function<void()>& settle,
+                          const std::function<void(const Op&)>& stream_op, uint64_t* launches, int* n_acc,
                           std::vector<JitPlan::Adj>* steps);
 // float registers keep the interpreter: their inner products are summed in FP64, which the compiled
 // passes would do in conversions
 inline bool run_adjoint_compiled(const std::vector<Op>&, float2*, float2*, int, double2*, unsigned, cudaStream_t,
-                                 const std::function<void(const Op&)>&, uint64_t*, int*, std::vector<JitPlan::Adj>*) {
+                                 const std::function<void()>&, const std::function<void(const Op&)>&, uint64_t*, int*,
+                                 std::vector<JitPlan::Adj>*) {
     return false;
 }
 

@@ -1265,18 +1265,31 @@ void adjoint_sweep(Handle* h, const std::vector<Cmd>& cmds, const DepTable& deps
         // stored psi', phi', so a step's inner product is conj(p_phi) p_psi <phi'|G|psi'>, with
         // p_psi and p_phi the products of f over the steps that ran before it, in the order the
         // tile passes run them (the planner reorders steps on disjoint qubits).  psi restarts
-        // from a checkpoint unscaled.
+        // from a checkpoint unscaled.  Compiled passes keep Im <phi|G|psi> alone, which a factor
+        // left out would turn: both states take theirs before a compiled segment (settle).
         c128 p_psi = 1.0, p_phi = 1.0;
         std::vector<Op> segment;
         auto stream_op = [&](const Op& o) {
             launch(h, o, psi);
             launch(h, o, phi);
         };
+        auto settle = [&]() {
+            auto take = [&](c128& f, vec2_t<T>* state) {
+                if (f == 1.0) return;
+                Op o;
+                o.kind = OP_SCALE;
+                o.m = {f};
+                launch(h, o, state);
+                f = 1.0;
+            };
+            take(p_psi, psi);
+            take(p_phi, phi);
+        };
         auto flush = [&]() {
             uint64_t launches = 0;
             std::vector<int> order;
-            if (compiled && run_adjoint_compiled(segment, psi, phi, n, acc_partials, nb, h->stream, stream_op, &launches,
-                                                 &n_acc, &compiled_steps)) {
+            if (compiled && run_adjoint_compiled(segment, psi, phi, n, acc_partials, nb, h->stream, settle, stream_op,
+                                                 &launches, &n_acc, &compiled_steps)) {
                 h->stats.launches += launches;
                 h->stats.passes += launches;
                 h->stats.hbm_bytes += launches * 4ull * h->dim() * h->amp_bytes();

@@ -81,3 +81,46 @@ def test_ansatz_layers_and_many_steps_on_few_qubits(restatement):
     cmds = [Command(ONE[int(rng.integers(4))], (int(rng.integers(4)),), (Param.symbol(nm),)) for nm in names]
     cmds = [Command(G.H, (q,)) for q in range(14)] + cmds
     _check(restatement, 14, cmds, {nm: float(v) for nm, v in zip(names, rng.uniform(-4, 4, 200))}, names)
+
+
+def _phase_rich(n, seed, segments, length, block_in):
+    """`segments` runs of `length` commands with many phase parameters; a fixed 4-qubit block, which the
+    compiled sweep refuses, in the middle of segment `block_in`."""
+    rng = np.random.default_rng([n, seed, block_in])
+    out, names = [], [f"t{k}" for k in range(18)]
+    for s in range(segments):
+        for i in range(length):
+            q = [int(x) for x in rng.permutation(n)[:4]]
+            p = Param.linear(float(rng.choice([-1.5, 1.0])), names[int(rng.integers(18))], float(rng.uniform(-1, 1)))
+            if s == block_in and i == length // 2:
+                z = rng.standard_normal((16, 16)) + 1j * rng.standard_normal((16, 16))
+                out.append(ir.custom(tuple(q), np.linalg.qr(z)[0]))
+            elif i % 5 == 4:
+                out.append(Command(G.CX, (q[0], q[1])))
+            else:
+                out.append(Command([G.Rz, G.Ry, G.P, G.Rx][i % 5], (q[0],), (p,)))
+    return out, {k: float(v) for k, v in zip(names, rng.uniform(-4, 4, 18))}, names
+
+
+# the tolerances of _check; the state a sweep leaves behind may lack a phase where it ends interpreted
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [14, 16])
+@pytest.mark.parametrize("block_in", [0, 1, 2])
+def test_segments_that_do_not_compile_beside_those_that_do(restatement, n, block_in, tmp_path, monkeypatch):
+    cmds, vals, names = _phase_rich(n, 21, 3, 30, block_in)
+    masks = observable.to_masks(circuits.tfim_chain(n) + circuits.random_pauli_sum(n, 12, seed=n, max_weight=3), n)
+    stream = ir.pack(cmds, vals, names)
+    want_e, want_g = restatement.adjoint(stream, n, len(names), masks)
+    monkeypatch.setenv("QSV_JIT_CACHE", str(tmp_path))
+    reg = Register(n)
+    reg.configure(1, 0, 3)
+    reg.set_checkpoint_interval(30)
+    for k in range(3):      # the forward sweep's segments, compiled before the reverse sweep's are counted
+        reg.apply(ir.pack(cmds[30 * k:30 * (k + 1)], vals))
+    reg.reset()
+    forward = len(list(tmp_path.iterdir()))
+    e, g = reg.adjoint(stream, len(names), masks)
+    reg.close()
+    assert len(list(tmp_path.iterdir())) > forward      # two of the three segments in compiled passes
+    assert abs(e - want_e) < 1e-10
+    np.testing.assert_allclose(g, want_g, atol=1e-9)
