@@ -30,7 +30,6 @@ constexpr int kFsWarpShots = 8;
 constexpr int kFsWarpBytes = 2 * 1024;          // always
 constexpr int kFsWarpBytesMany = 8 * 1024;      // with shots for every multiprocessor's block
 constexpr int kFsWarpBytesNoise = 16 * 1024;    // the same, plans with noise
-constexpr size_t kFsWarpMax = 224 * 1024;       // one block's shared memory
 constexpr int kFsNarrowBytes = 16 * 1024;   // registers up to here: 128 threads a CTA, else 256
 constexpr int kFsMaxCoef = 512;          // doubles of one step's coefficients (a 4-qubit block)
 constexpr int kFsMtBytes = 4 * 624 + 16; // one MT19937 state, padded to keep the plan aligned
@@ -776,8 +775,15 @@ bool run_trajectories_fused(const TrPlan& plan, int n, const vec2_t<T>* d_prefix
     for (const FsStep& f : steps) noise |= f.kind == FS_PAULI_NOISE || f.kind == FS_KRAUS_NOISE;
     const bool many = n_shots >= static_cast<size_t>(kFsWarpShots) * static_cast<size_t>(sms);
     const int warp_bytes = !many ? kFsWarpBytes : noise ? kFsWarpBytesNoise : kFsWarpBytesMany;
-    const bool warps = amp_bytes <= static_cast<size_t>(warp_bytes) &&
-                       kFsWarpShots * shot_area + prog_bytes <= kFsWarpMax;
+    // eight shots and their plan take what one block may have beside the kernel's own shared memory
+    bool warps = amp_bytes <= static_cast<size_t>(warp_bytes);
+    if (warps) {
+        int block_max = 0;
+        check_cuda(cudaDeviceGetAttribute(&block_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "block shared memory");
+        cudaFuncAttributes own{};
+        check_cuda(cudaFuncGetAttributes(&own, k_fs_run<T, 32, kFsWarpShots>), "fused trajectory kernel");
+        warps = kFsWarpShots * shot_area + prog_bytes + own.sharedSizeBytes <= static_cast<size_t>(block_max);
+    }
     const int resident = warps || shot_area + prog_bytes <= kFsResidentMax ? 1 : 0;
     const int per_cta = warps ? kFsWarpShots : 1;
     const size_t smem = per_cta * shot_area + (resident ? prog_bytes : kFsMaxCoef * sizeof(double));

@@ -106,3 +106,29 @@ def test_engine_generations(n):
     finally:
         reg.close()
     np.testing.assert_array_equal(regs, want)
+
+
+@pytest.mark.parametrize("n,noisy,around", [(10, True, 441), (9, False, 815)])
+def test_plans_that_just_fill_a_block(n, noisy, around):
+    """Gates under alternating conditions (a step of 176 bytes each: a record and a 2 x 2 matrix), as many
+    as fill a block's shared memory beside eight shots, and a few more and fewer: each plan runs, with
+    the outcomes of the executor that keeps its shots in device memory."""
+    from openqarp_b200 import NoiseModel
+    shots, seed, G = 1300, 5, GateType
+    for count in range(around - 10, around + 11):
+        cmds = [Command(G.H, (q,)) for q in range(n)] + [Command(G.U, (0,), (0.7, 0.1, 0.4)),
+                                                        Command(G.Measure, (0,), (), None, (0,))]
+        cmds += [Command(G.X, (1 + i % (n - 1),), (), None, (), (0,), (i % 2 == 0,)) for i in range(count)]
+        buf, got = ir.pack(cmds).buf, []
+        for batch in (0, 512):
+            reg = Register(n)
+            try:
+                reg.set_trajectory_batch(batch)
+                if noisy:
+                    reg.set_noise(NoiseModel.amplitude_damping(0.2, ["U"]))
+                got.append(reg.run_trajectories(buf, seed, shots)[:2])
+            finally:
+                reg.close()
+        np.testing.assert_array_equal(got[0][1], got[1][1])
+        # a draw within rounding of a running sum may fall to either side
+        assert np.mean(got[0][0] == got[1][0]) > 0.998, count
