@@ -176,6 +176,9 @@ c128 unit_phase(c128 v) {
     return a > 0 ? v / a : c128(1.0, 0.0);
 }
 
+// Whether v is a phase: products of a few thousand gates' phases stay well inside.
+bool is_phase(c128 v) { return std::abs(std::norm(v) - 1.0) <= 1e-10; }
+
 Factor1q factor_1q(const std::vector<c128>& u) {
     Factor1q f;
     double c = std::abs(u[0]), s = std::abs(u[2]);
@@ -756,11 +759,13 @@ struct Gen {
         uint32_t tm = 0;
         for (int b = 0; b < op.k; ++b)
             if (turned_q(static_cast<int>(op.qubits[b]))) tm |= 1u << b;
-        if (op.k == 1) {
+        // a one-qubit diagonal of phases is owed; any other (a projector, say) keeps its table: tables of
+        // owed pairs divide by the first entry and count on moduli near 1
+        if (op.k == 1 && is_phase(op.m[0]) && is_phase(op.m[1])) {
             const int q = static_cast<int>(op.qubits[0]);
             c128* p = owed(q);
             for (uint32_t v = 0; v < 2; ++v) p[v] *= op.m[v ^ tm];
-            mark(0xE1u, static_cast<uint64_t>(q));
+            mark(0xEFu, static_cast<uint64_t>(q));
             return;
         }
         const size_t at = coef.size();

@@ -46,3 +46,25 @@ def test_turned_bits_match_oracle(restatement, n, k, dtype, tol):
         reg.apply(buf)
         assert np.max(np.abs(reg.get_state() - want)) < tol
         reg.close()
+
+
+# one-qubit diagonals that are no phases (projectors, weights), on places of every kind, beside phases
+# and turned bits, after the same circuit with a phase there: a hundred products of amplitudes below 1
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,tol", [("complex128", 1e-12), ("complex64", 2e-5)])
+@pytest.mark.parametrize("d", [(1.0, 1.0j), (0.0, 1.0), (1.0, 0.0), (0.0, 0.0), (0.25, 1.0), (-0.5j, 1e-30)])
+def test_diagonals_of_any_modulus(restatement, d, dtype, tol):
+    n, rng = 14, np.random.default_rng(8)
+    for places in ([0], [5], [12, 13], list(range(n))):
+        cmds = [Command(G.Ry, (q,), (float(rng.uniform(-7, 7)),)) for q in range(n)]
+        for q in places:
+            cmds += [Command(G.Rz, (q,), (0.3 + q,)), ir.custom((q,), np.diag(d)), Command(G.CZ, (q, (q + 1) % n)),
+                     Command(G.Rx, ((q + 3) % n,), (4.0 - q,))]
+        cmds += [Command(G.Ry, (q,), (float(rng.uniform(-7, 7)),)) for q in range(n)]
+        buf = ir.pack(cmds).buf
+        want = restatement.statevector(buf, n)
+        reg = Register(n, dtype)
+        reg.configure(0, 0, 3, 12)
+        reg.apply(buf)
+        assert np.max(np.abs(reg.get_state() - want)) < tol, places     # NaN fails too
+        reg.close()
