@@ -179,7 +179,8 @@ c128 unit_phase(c128 v) {
 // Whether v is a phase: products of a few thousand gates' phases stay well inside.
 bool is_phase(c128 v) { return std::abs(std::norm(v) - 1.0) <= 1e-10; }
 
-Factor1q factor_1q(const std::vector<c128>& u) {
+// False where u is not unitary (to 1e-12 an entry).
+bool factor_unitary(const std::vector<c128>& u, Factor1q* out) {
     Factor1q f;
     double c = std::abs(u[0]), s = std::abs(u[2]);
     const double r = std::sqrt(c * c + s * s);
@@ -197,11 +198,18 @@ Factor1q factor_1q(const std::vector<c128>& u) {
         f.d1[0] = P; f.d1[1] = unit_phase(u[2]) / R;
         f.d2[0] = R; f.d2[1] = c128(1.0, 0.0);
     }
-    // the factors must reproduce the gate: a planner or rounding surprise becomes a host error
     const c128 m[4] = {c * f.d1[0] * f.d2[0], -s * f.d1[0] * f.d2[1], s * f.d1[1] * f.d2[0], c * f.d1[1] * f.d2[1]};
     for (int e = 0; e < 4; ++e)
-        if (std::abs(m[e] - u[e]) > 1e-12 * std::max(1.0, std::abs(u[e])))
-            throw std::logic_error("JIT tiles: one-qubit factorisation does not reproduce the gate");
+        if (std::abs(m[e] - u[e]) > 1e-12 * std::max(1.0, std::abs(u[e]))) return false;
+    *out = f;
+    return true;
+}
+
+// the factors must reproduce the gate: a planner or rounding surprise becomes a host error
+Factor1q factor_1q(const std::vector<c128>& u) {
+    Factor1q f;
+    if (!factor_unitary(u, &f))
+        throw std::logic_error("JIT tiles: one-qubit factorisation does not reproduce the gate");
     return f;
 }
 
@@ -1029,6 +1037,9 @@ struct Gen {
                                            m[0] == m[3] && m[1] == -m[2];
                 mark(0xAD5u, real_rotation ? 1u : 0u);
                 if (!real_rotation) {
+                    // a matrix given to fewer digits than these passes factor by: the interpreted sweep's
+                    Factor1q f;
+                    if (!factor_unitary(m, &f)) return false;
                     complex_gates.push_back(st);
                     continue;
                 }

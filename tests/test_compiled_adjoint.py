@@ -124,3 +124,25 @@ def test_segments_that_do_not_compile_beside_those_that_do(restatement, n, block
     assert len(list(tmp_path.iterdir())) > forward      # two of the three segments in compiled passes
     assert abs(e - want_e) < 1e-10
     np.testing.assert_allclose(g, want_g, atol=1e-9)
+
+
+# matrices rounded to 32 bits are unitary to 1e-7: the sweep that applies them as they are, the tolerances of _check
+@pytest.mark.gpu
+def test_matrices_of_fewer_digits(restatement):
+    n = 14
+    rng = np.random.default_rng(31)
+    cmds, vals, names = _circuit(n, 7, 40)
+    for q in range(0, n, 3):
+        z = np.linalg.qr(rng.standard_normal((2, 2)) + 1j * rng.standard_normal((2, 2)))[0]
+        at = 12 + 2 * q
+        # the forward sweep takes it within a two-qubit block
+        cmds[at:at] = [ir.custom((q,), z.astype(np.complex64)), Command(G.CX, (q, (q + 1) % n))]
+    masks = observable.to_masks(circuits.tfim_chain(n), n)
+    stream = ir.pack(cmds, vals, names)
+    want_e, want_g = restatement.adjoint(stream, n, len(names), masks)
+    reg = Register(n)
+    reg.configure(2, 0, 3)
+    e, g = reg.adjoint(stream, len(names), masks)
+    reg.close()
+    assert abs(e - want_e) < 1e-10
+    np.testing.assert_allclose(g, want_g, atol=1e-9)
