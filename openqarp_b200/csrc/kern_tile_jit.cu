@@ -1028,13 +1028,15 @@ struct Gen {
             for (int p = 0; p < kRtRegBits; ++p) bit_of_slot[p] = L.reg[p];
             for (const RtStep* st : heads) {
                 const std::vector<c128>& m = st->op->m;
+                // by the gate's kind, not its entries: an X rotation by 0 has real ones too, and a structure
+                // is compiled once for all angles
+                bool real_rotation = st->op->y_turn;
                 if (st->kind == RT_ADJ) {
                     const AdjKind kind = adj_kind(*st->op);
                     if (kind != ADJ_X && kind != ADJ_Y) return false;
                     adj_off(*st, L, kind);
+                    real_rotation = kind == ADJ_Y;
                 }
-                const bool real_rotation = m[0].imag() == 0 && m[1].imag() == 0 && m[2].imag() == 0 && m[3].imag() == 0 &&
-                                           m[0] == m[3] && m[1] == -m[2];
                 mark(0xAD5u, real_rotation ? 1u : 0u);
                 if (!real_rotation) {
                     // a matrix given to fewer digits than these passes factor by: the interpreted sweep's

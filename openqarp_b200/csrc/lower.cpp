@@ -207,7 +207,11 @@ std::vector<Op> lower(const Cmd& c, int n) {
         case X: case Y: case H: case SX: case SXDG:
             return {make_dense1(c.q[0], fixed(g))};
         case RX: return {make_dense1(c.q[0], m_rx(param(c, 0)))};
-        case RY: return {make_dense1(c.q[0], m_ry(param(c, 0)))};
+        case RY: {
+            Op o = make_dense1(c.q[0], m_ry(param(c, 0)));
+            o.y_turn = true;
+            return {o};
+        }
         case U: return {make_dense1(c.q[0], m_u(param(c, 0), param(c, 1), param(c, 2)))};
         case Z: case S: case SDG: case T: case TDG:
             return {make_phase(bit(c.q[0]), fixed(g)[3])};

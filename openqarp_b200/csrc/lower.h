@@ -99,6 +99,7 @@ struct Op {
     uint64_t mask = 0, zmask = 0;
     uint64_t ctrl = 0;             // OP_DENSE: control bits (all must be 1)
     int target = 0;
+    bool y_turn = false;           // OP_DENSE of a Y rotation: [[c, -s], [s, c]] at every angle
     std::vector<c128> m;
     std::vector<uint64_t> table;   // OP_PERM
     std::vector<uint32_t> pq;      // OP_PERM qubits (may exceed 8)

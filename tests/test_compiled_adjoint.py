@@ -146,3 +146,41 @@ def test_matrices_of_fewer_digits(restatement):
     reg.close()
     assert abs(e - want_e) < 1e-10
     np.testing.assert_allclose(g, want_g, atol=1e-9)
+
+
+# a structure is compiled once for all angles: zeros (all of them, or some) compile nothing new
+@pytest.mark.gpu
+def test_angles_of_zero_compile_nothing(restatement, tmp_path, monkeypatch):
+    n = 15
+    names = [f"t{k}" for k in range(12)]
+    fixed = [f"f{k}" for k in range(4)]
+    rng = np.random.default_rng(41)
+    cmds = []
+    for i in range(90):
+        q = [int(x) for x in rng.permutation(n)[:2]]
+        sym = Param.symbol(names[int(rng.integers(12))])
+        pick = i % 9
+        if pick < 4:
+            cmds.append(Command(ONE[pick], (q[0],), (sym,)))
+        elif pick < 6:
+            cmds.append(Command([G.Rx, G.Ry][pick - 4], (q[0],), (Param.symbol(fixed[int(rng.integers(4))]),)))
+        elif pick < 8:
+            cmds.append(Command(TWO[int(rng.integers(7))], (q[0], q[1]), (sym,)))
+        else:
+            cmds.append(Command(G.CX, (q[0], q[1])))
+    masks = observable.to_masks(circuits.tfim_chain(n), n)
+    monkeypatch.setenv("QSV_JIT_CACHE", str(tmp_path))
+    reg = Register(n)
+    reg.configure(0, 0, 3)
+    files = 0
+    for zero in (0.0, 0.5, 1.0):       # share of the angles that are 0
+        vals = {k: 0.0 if rng.random() < zero else float(rng.uniform(-4, 4)) for k in names + fixed}
+        stream = ir.pack(cmds, vals, names)
+        want_e, want_g = restatement.adjoint(stream, n, len(names), masks)
+        reg.reset()
+        e, g = reg.adjoint(stream, len(names), masks)
+        assert abs(e - want_e) < 1e-10
+        np.testing.assert_allclose(g, want_g, atol=1e-9)
+        files = files or len(list(tmp_path.iterdir()))
+        assert len(list(tmp_path.iterdir())) == files > 0, zero
+    reg.close()
