@@ -39,6 +39,7 @@
 #include <cuda.h>
 #include <nvrtc.h>
 
+#include "../../include/qsv.h"
 #include "kernels.h"
 #include "tile.h"
 
@@ -254,6 +255,9 @@ struct Gen {
     int normalised = 0;   // normalised tables since cglob was last applied
     double flops = 0;   // FP64 operations per thread per tile (FMA = 2, MUL = 1)
 
+    // Coefficients come in pairs, real ones with a 0 beside them: a complex entry that straddles 16
+    // bytes is read in halves, and ptxas then spills amplitudes (28-qubit brickwork in complex128: 2680
+    // bytes of spill stores over its 15 passes against 1150, 48.7 against 47.1 ms; 656 as it is now).
     size_t push(c128 v) {
         coef.push_back(v.real());
         coef.push_back(v.imag());
@@ -508,8 +512,7 @@ struct Gen {
     void rotate(int p, int b, double c, double s, c128 d0, c128 d1) {
         const bool cos_form = std::abs(c) >= std::abs(s);
         double scale = cos_form ? c : s;
-        const size_t at = coef.size();
-        coef.push_back(cos_form ? s / c : -(c / s));
+        const size_t at = push(cos_form ? s / c : -(c / s));
         if (pair) {
             cglob *= scale;
             scale = 1.0;
@@ -549,8 +552,7 @@ struct Gen {
     // form the host cannot rewrite.
     void unturn_slot(const RtLayout& L, int p) {
         const int b = L.reg[p];
-        const size_t at = coef.size();
-        coef.push_back(turned[b] ? 1.0 : 0.0);
+        const size_t at = push(turned[b] ? 1.0 : 0.0);
         if (turned[b]) std::swap(pend[b][0], pend[b][1]);
         turned[b] = false;
         mark(0xF7u, static_cast<uint64_t>(p));
@@ -694,8 +696,7 @@ struct Gen {
                 *rm |= 1u << k;
                 continue;
             }
-            const size_t at = coef.size();
-            coef.push_back(turned[b] ? 1.0 : 0.0);
+            const size_t at = push(turned[b] ? 1.0 : 0.0);
             c += (c.empty() ? "" : " && ") + std::string(w == 'l' ? "((((lane >> " : "((((warp >> ") + std::to_string(k) +
                  ") & 1u) != 0u) != (" + cr(at) + " != 0))";
         }
@@ -1104,8 +1105,8 @@ __device__ __forceinline__ double flip(double a, int m) {
 }
 __device__ __forceinline__ float flip(float a, int m) { return __int_as_float(__float_as_int(a) ^ m); }
 // the bits of i placed at the set bits of m, lowest first
-__device__ __forceinline__ u64 spread(u64 i, u64 m) {
-    u64 r = 0;
+__device__ __forceinline__ unsigned spread(unsigned i, unsigned m) {
+    unsigned r = 0;
     for (; i && m; i >>= 1, m &= m - 1)
         if (i & 1) r |= m & (0 - m);
     return r;
@@ -1130,7 +1131,7 @@ constexpr bool kJitDebug = true;
 const char* kPreludeDebug = "";
 constexpr bool kJitDebug = false;
 #endif
-
+static_assert(kRtRegBits == 4, "JitStore::step and the kernels' d0..d3");
 
 // Walk one pass's plan: coefficients, structural signature and (with emit) the steps' source.
 // Returns false when the pass needs an op the generator does not handle or too many
@@ -1280,8 +1281,8 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
             size_t e = j;
             while (e + 1 < outside.size() &&
                    outside[e + 1] - static_cast<int>(e + 1) == outside[j] - static_cast<int>(j)) ++e;
-            const uint64_t mask = ((e - j + 1) >= 64 ? ~0ull : ((1ull << (e - j + 1)) - 1)) << j;
-            base += std::string(" | ((") + var + " & " + hex64(mask) + ") << " + std::to_string(outside[j] - static_cast<int>(j)) + ")";
+            const uint32_t mask = ((1u << (e - j + 1)) - 1u) << j;
+            base += std::string(" | ((u64)(") + var + " & " + std::to_string(mask) + "u) << " + std::to_string(outside[j] - static_cast<int>(j)) + ")";
             j = e + 1;
         }
         return base;
@@ -1317,12 +1318,6 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
         }
         return x.str();
     };
-    // per register slot of the store: the step to the amplitude with that bit set
-    std::string strides;
-    for (int p = 0; p < kRtRegBits && !kJitDebug && !f32; ++p) {
-        const std::string q = std::to_string(tq[F.reg[p]]);
-        strides += "  const long long d" + std::to_string(p) + " = (turned >> " + q + ") & 1 ? -(1ll << " + q + ") : 1ll << " + q + ";\n";
-    }
     std::ostringstream s;
     if (f32) {
         s << "typedef float R; typedef float2 R2;\n#define FMA fmaf\n#define MK make_float2\n";
@@ -1332,7 +1327,8 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
     }
     s << "struct __align__(8) C" << idx << " { R c[" << nc << "]; };\n"
       << "extern \"C\" __global__ void __launch_bounds__(" << kJitThreads << ", " << (pair ? 1 : jit_ctas(f32))
-      << ") qsv_jit_" << idx << "(R2* __restrict__ s, u64 n_tiles, u64 tmask, u64 tstep, u64 turned, "
+      << ") qsv_jit_" << idx << "(R2* __restrict__ s, unsigned n_tiles, unsigned tmask, unsigned tstep, u64 turned, "
+      << (kJitDebug ? "" : "long long d0, long long d1, long long d2, long long d3, ")
       << (pair ? "R2* __restrict__ s2, double2* __restrict__ partials, " : "") << "const __grid_constant__ C" << idx << " P"
       << (kJitDebug ? ", unsigned long long* __restrict__ dbg" : "") << ") {\n"
       << "  extern __shared__ __align__(16) unsigned char smem[];\n"
@@ -1348,8 +1344,7 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
       << "  const u64 gfin = " << gfin << ";\n"
       // the i-th tile is the i-th subset of tmask; tstep = spread(gridDim.x, tmask), added with the
       // carries running through the other bits
-      << "  u64 i = blockIdx.x, t = spread(i, tmask);\n"
-      << strides
+      << "  unsigned i = blockIdx.x, t = spread(i, tmask);\n"
       << "  if (i < n_tiles) {\n    const u64 b0 = " << deposit("t") << ";\n" << issue("b0") << "  }\n"
       << "  asm volatile(\"cp.async.commit_group;\\n\" ::: \"memory\");\n"
       << "  for (; i < n_tiles; i += gridDim.x, t = ((t | ~tmask) + tstep) & tmask) {\n"
@@ -1377,11 +1372,11 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
     s << "  }\n  __syncthreads();\n"
       << steps
       << "  __syncthreads();\n"
-      << "  if (i + gridDim.x < n_tiles) {\n    const u64 tn = ((t | ~tmask) + tstep) & tmask;\n    const u64 b1 = " << deposit("tn")
+      << "  if (i + gridDim.x < n_tiles) {\n    const unsigned tn = ((t | ~tmask) + tstep) & tmask;\n    const u64 b1 = " << deposit("tn")
       << ";\n" << issue("b1") << "  }\n"
       << "  asm volatile(\"cp.async.commit_group;\\n\" ::: \"memory\");\n";
     s << "  const u64 to = (base | gfin) ^ turned;\n";
-    for (int r = 0; r < kJitAmps && (kJitDebug || f32); ++r) {
+    for (int r = 0; kJitDebug && r < kJitAmps; ++r) {
         uint64_t gc = 0;
         for (int p = 0; p < kRtRegBits; ++p)
             if ((r >> p) & 1) gc |= 1ull << tq[F.reg[p]];
@@ -1389,11 +1384,12 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
             s << "  __stcs(" << (set == 'a' ? "s" : "s2") << " + " << at("to ^ " + hex64(gc)) << ", MK(" << re(set, r) << ", "
               << im(set, r) << "));\n";
     }
-    // Complex128: the slots in Gray order, a pointer stepping by a slot bit's stride, negative where
-    // the bit is turned.  An XOR and a scaled address per store were 3 % of a pass's instructions: 28
-    // qubits, depth 20, 48.3 -> 47.4 ms.  (Complex64, FP32 issue in two-amplitude words: 24.34 against
-    // 24.39, so it keeps the XOR.)
-    if (!kJitDebug && !f32) {
+    // The slots in Gray order, a pointer stepping by a slot bit's stride, negative where the bit is turned
+    // (the debug build checks an index per store instead).  The strides are kernel parameters and tile
+    // numbers 32-bit: formed in the kernel and 64-bit they took the registers that the amplitudes need
+    // (28 qubits, depth 20, complex128: 47.1 -> 46.3 ms applied again and again; an XOR and a scaled
+    // address per store 47.3).
+    if (!kJitDebug) {
         for (char set : sets) s << "  R2* w" << set << " = " << (set == 'a' ? "s" : "s2") << " + to;\n";
         for (int k = 0, r = 0; k < kJitAmps; ++k) {
             for (char set : sets) s << "  __stcs(w" << set << ", MK(" << re(set, r) << ", " << im(set, r) << "));\n";
@@ -1416,7 +1412,7 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
 // Source (with emit) or only the signature and coefficients (without) of one pass; `pair`: a pass of the
 // reverse sweep, with its adjoint steps' results in `outs`.
 bool gen_pass(const TilePass& pass, const RtPlan& plan, int n, int idx, bool emit, bool f32, bool pair, std::string* src,
-              std::vector<double>* coef, uint64_t* sig_hash, uint64_t* turned, double* flops_per_amp = nullptr,
+              std::vector<double>* coef, uint64_t* sig_hash, JitStore* store, double* flops_per_amp = nullptr,
               const Carry* cin = nullptr, bool final = true, Carry* cout = nullptr, std::vector<Gen::AdjOut>* outs = nullptr,
               int* n_acc = nullptr) {
     Gen g;
@@ -1425,7 +1421,11 @@ bool gen_pass(const TilePass& pass, const RtPlan& plan, int n, int idx, bool emi
     g.pair = pair;
     g.mark(pair ? 0xFADu : f32 ? 0xF32u : 0xF64u);
     RtLayout last{};
-    if (!walk_pass(pass, plan, n, &g, &last, cin, final, cout, turned)) return false;
+    if (!walk_pass(pass, plan, n, &g, &last, cin, final, cout, &store->turned)) return false;
+    for (int p = 0; p < kRtRegBits; ++p) {
+        const uint32_t q = pass.tile_qubits[last.reg[p]];
+        store->step[p] = (store->turned >> q) & 1 ? -(1ll << q) : 1ll << q;
+    }
     if (g.n_acc > kPairMaxAcc) return false;
     uint64_t h = 1469598103934665603ull;
     for (uint64_t v : g.sig)
@@ -1520,7 +1520,7 @@ struct PassWalk {
     bool has_cin = false;
     Carry cin;
     bool final = true;
-    uint64_t turned = 0;  // qubits the store turns back (walk_pass)
+    JitStore store;
     std::vector<Gen::AdjOut> outs;
     int n_acc = 0;
 };
@@ -1535,7 +1535,7 @@ std::vector<PassWalk> walk_all(const std::vector<const TilePass*>& passes, std::
         if (!plan_rt(*passes[i], &plans[i], f32 ? 8 : 16)) continue;
         std::string unused;
         PassWalk& w = alone[i];
-        w.ok = gen_pass(*passes[i], plans[i], n, 0, false, f32, pair, &unused, &w.coef, &w.sig, &w.turned,
+        w.ok = gen_pass(*passes[i], plans[i], n, 0, false, f32, pair, &unused, &w.coef, &w.sig, &w.store,
                         &w.flops_per_amp, nullptr, true, nullptr, &w.outs, &w.n_acc);
     }
     std::vector<PassWalk> chained(np);
@@ -1552,7 +1552,7 @@ std::vector<PassWalk> walk_all(const std::vector<const TilePass*>& passes, std::
         if (in_chain) w.cin = cur;
         Carry next;
         std::string unused;
-        w.ok = gen_pass(*passes[i], plans[i], n, 0, false, f32, pair, &unused, &w.coef, &w.sig, &w.turned,
+        w.ok = gen_pass(*passes[i], plans[i], n, 0, false, f32, pair, &unused, &w.coef, &w.sig, &w.store,
                         &w.flops_per_amp, w.has_cin ? &w.cin : nullptr, w.final, w.final ? nullptr : &next, &w.outs, &w.n_acc);
         if (!w.ok) return alone;
         cur = std::move(next);
@@ -1634,7 +1634,7 @@ JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int devic
         if (!w.ok && pair && !passes[i]->tile_qubits.empty()) return JitPlan{};   // all of a sweep, or none
         if (!w.ok) continue;
         out.flops_per_amp.push_back(w.flops_per_amp);
-        out.turned.push_back(w.turned);
+        out.store.push_back(w.store);
         out.n_acc.push_back(w.n_acc);
         for (Gen::AdjOut& a : w.outs) {
             for (auto& [acc, weight] : a.acc) acc += out.total_acc;
@@ -1673,9 +1673,10 @@ JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int devic
             const size_t i = pass_of[missing[j]];
             const PassWalk& w = walks[i];
             std::vector<double> coef;
-            uint64_t sig = 0, turned = 0;
+            uint64_t sig = 0;
+            JitStore store;
             Carry next;
-            gen_pass(*passes[i], plans[i], n, 0, true, f32, pair, &srcs[j], &coef, &sig, &turned, nullptr,
+            gen_pass(*passes[i], plans[i], n, 0, true, f32, pair, &srcs[j], &coef, &sig, &store, nullptr,
                      w.has_cin ? &w.cin : nullptr, w.final, w.final ? nullptr : &next);
             srcs[j] = std::string(kPrelude) + kPreludeDebug + srcs[j] + tag;
             char name[40];
@@ -1720,25 +1721,29 @@ JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int devic
 }
 
 namespace {
-void launch_pass(const JitPlan& plan, int pass, void* s, void* s2, double2* partials, int n, unsigned long long tmask,
+void launch_pass(const JitPlan& plan, int pass, void* s, void* s2, double2* partials, int n, uint64_t tiles,
                  cudaStream_t st) {
     const int k = plan.idx.at(pass);
     if (k < 0) throw std::logic_error("JIT tiles: pass was not compiled");
     int sms = 0, device = 0;
     check_cuda(cudaGetDevice(&device), "device");
     check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "sm count");
-    tmask &= (1ull << (n - kRtQubits)) - 1;
-    unsigned long long n_tiles = 1ull << __builtin_popcountll(tmask);
+    // tile numbers take n - 12 bits
+    static_assert(QSV_MAX_QUBITS - kRtQubits < 32, "tile numbers are 32-bit in the kernels");
+    unsigned tmask = static_cast<unsigned>(tiles & ((1ull << (n - kRtQubits)) - 1));
+    unsigned n_tiles = 1u << __builtin_popcount(tmask);
     const int ctas = plan.pair ? 1 : jit_ctas(plan.f32);
     const unsigned grid = static_cast<unsigned>(
-        std::min<unsigned long long>(n_tiles, static_cast<unsigned long long>(ctas) * sms));
+        std::min<uint64_t>(n_tiles, static_cast<uint64_t>(ctas) * static_cast<uint64_t>(sms)));
     const std::vector<uint8_t>& c = plan.coef[static_cast<size_t>(k)];
-    unsigned long long turned = plan.turned[static_cast<size_t>(k)];
-    unsigned long long tstep = 0;      // spread(grid, tmask)
-    for (unsigned long long i = grid, m = tmask; i && m; i >>= 1, m &= m - 1)
+    JitStore store = plan.store[static_cast<size_t>(k)];
+    unsigned tstep = 0;      // spread(grid, tmask)
+    for (unsigned i = grid, m = tmask; i && m; i >>= 1, m &= m - 1)
         if (i & 1) tstep |= m & (0 - m);
     double2* part = partials ? partials + static_cast<size_t>(plan.acc0[static_cast<size_t>(k)]) * grid : nullptr;
-    std::vector<void*> args{&s, &n_tiles, &tmask, &tstep, &turned};
+    std::vector<void*> args{&s, &n_tiles, &tmask, &tstep, &store.turned};
+    if (!kJitDebug)
+        for (long long& d : store.step) args.push_back(&d);
     if (plan.pair) args.insert(args.end(), {static_cast<void*>(&s2), static_cast<void*>(&part)});
     args.push_back(const_cast<uint8_t*>(c.data()));
 #ifdef QSV_DEBUG_BOUNDS
@@ -1830,9 +1835,10 @@ std::string jit_source_for_test(const std::vector<const TilePass*>& passes, int 
         if (!w.ok) continue;
         std::string ps;
         std::vector<double> coef;
-        uint64_t sig = 0, turned = 0;
+        uint64_t sig = 0;
+        JitStore store;
         Carry out;
-        if (!gen_pass(*passes[i], plans[i], n, next, true, f32, false, &ps, &coef, &sig, &turned, nullptr,
+        if (!gen_pass(*passes[i], plans[i], n, next, true, f32, false, &ps, &coef, &sig, &store, nullptr,
                       w.has_cin ? &w.cin : nullptr, w.final, w.final ? nullptr : &out))
             continue;
         if (next > 0) {

@@ -161,6 +161,12 @@ double run_tiled(const std::vector<TilePass>& passes, vec2_t<T>* s, int n, cudaS
                  uint64_t support = ~0ull);
 
 // ---------------------------------------------------------------- JIT register tiles (kern_tile_jit.cu)
+// The store of a compiled pass: the qubits whose bits it flips, and from an amplitude with a register-slot
+// bit clear to the one with it set (backwards where the bit is flipped).
+struct JitStore {
+    uint64_t turned = 0;
+    long long step[4] = {};
+};
 // The register-tile passes of a stream compiled to straight-line kernels.
 struct JitPlan {
     bool f32 = false;                       // complex64 storage
@@ -168,7 +174,7 @@ struct JitPlan {
     std::vector<int> idx;                   // per pass: kernel index, -1 = not compiled
     std::vector<std::vector<uint8_t>> coef; // per kernel: its coefficients (kernel parameters)
     std::vector<void*> fns;                 // per kernel: the loaded function (CUfunction)
-    std::vector<uint64_t> turned;           // per kernel: qubits whose bits the store flips (kernel parameter)
+    std::vector<JitStore> store;            // per kernel: where its stores go (kernel parameters)
     std::vector<double> flops_per_amp;      // per kernel: FP64 operations per amplitude (FMA = 2)
     // pair plans: accumulators per kernel and before it, and each adjoint step's Im <phi|G|psi> as a
     // weighted sum of accumulators, by the step's slot

@@ -68,3 +68,22 @@ def test_diagonals_of_any_modulus(restatement, d, dtype, tol):
         reg.apply(buf)
         assert np.max(np.abs(reg.get_state() - want)) < tol, places     # NaN fails too
         reg.close()
+
+
+# what every pass reads of its coefficients is a whole pair (no device needed: the source is looked at)
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_coefficients_come_in_pairs(dtype, tmp_path, monkeypatch):
+    import ctypes
+    import re
+    from openqarp_b200._lib import check, lib, u8ptr
+    monkeypatch.setenv("QSV_JIT_DUMP", str(tmp_path / "passes.cu"))
+    buf = ir.pack(_circuit(15, 4, 60)).buf
+    passes, kernels, size = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_uint64()
+    check(lib.qsv_jit_check(u8ptr(buf), len(buf), 15, dtype, 0, 0, 10, 0, ctypes.byref(passes), ctypes.byref(kernels),
+                            ctypes.byref(size)))
+    src = (tmp_path / "passes.cu").read_text()
+    singles = re.findall(r"const R t = P\.c\[(\d+)\]|\(P\.c\[(\d+)\] != 0\)", src)
+    products = re.findall(r"= P\.c\[(\d+)\] \* xr - P\.c\[(\d+)\] \* xi", src)
+    assert len(singles) > 20 and len(products) > 100
+    assert all(int(a or b) % 2 == 0 for a, b in singles)
+    assert all(int(a) % 2 == 0 and int(b) == int(a) + 1 for a, b in products)
