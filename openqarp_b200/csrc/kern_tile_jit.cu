@@ -1732,9 +1732,10 @@ void launch_pass(const JitPlan& plan, int pass, void* s, void* s2, double2* part
     static_assert(QSV_MAX_QUBITS - kRtQubits < 32, "tile numbers are 32-bit in the kernels");
     unsigned tmask = static_cast<unsigned>(tiles & ((1ull << (n - kRtQubits)) - 1));
     unsigned n_tiles = 1u << __builtin_popcount(tmask);
-    const int ctas = plan.pair ? 1 : jit_ctas(plan.f32);
-    const unsigned grid = static_cast<unsigned>(
-        std::min<uint64_t>(n_tiles, static_cast<uint64_t>(ctas) * static_cast<uint64_t>(sms)));
+    // a pair pass writes its partials by block: the grid its caller sized them for
+    const unsigned grid = plan.pair ? adjoint_tile_grid(n, kRtQubits)
+                                    : static_cast<unsigned>(std::min<uint64_t>(
+                                          n_tiles, static_cast<uint64_t>(jit_ctas(plan.f32)) * static_cast<uint64_t>(sms)));
     const std::vector<uint8_t>& c = plan.coef[static_cast<size_t>(k)];
     JitStore store = plan.store[static_cast<size_t>(k)];
     unsigned tstep = 0;      // spread(grid, tmask)
@@ -1770,6 +1771,7 @@ bool run_adjoint_compiled(const std::vector<Op>& ops, double2* psi, double2* phi
                           const std::function<void(const Op&)>& stream_op, uint64_t* launches, int* n_acc,
                           std::vector<JitPlan::Adj>* steps) {
     if (ops.empty()) return true;
+    if (nb != adjoint_tile_grid(n, kRtQubits)) throw std::logic_error("adjoint partials sized for another grid");
     // a pass ends where its accumulators or its parameters would overflow (at most 32 doubles of phase
     // table and ratio a step, or the step's matrix)
     std::vector<TilePass> passes;

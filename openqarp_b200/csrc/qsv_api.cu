@@ -1249,6 +1249,7 @@ void adjoint_sweep(Handle* h, const std::vector<Cmd>& cmds, const DepTable& deps
     // tiled: the reverse stream runs as tile passes over both states, several reverse steps a
     // pass; narrower registers take one launch per reverse step
     const unsigned nb = tiled ? adjoint_tile_grid(n, mt) : adjoint_blocks(n);
+    static_assert(adjoint_tile_qubits<double>() == kRtQubits, "interpreted and compiled passes share one partial per block");
     // compiled pair passes where the forward sweep's passes are compiled too (executor 3), so a structure's
     // first call is the only one to wait for a compiler: the 24-qubit, 384-parameter reverse sweep takes
     // 6.3 ms in 18 of them and 30.5 ms in 19 interpreted passes
