@@ -36,6 +36,7 @@ namespace {
 constexpr int kQThreads = 512;
 constexpr int kQMaxEdges = 96;
 constexpr int kQMaxQubits = 24;
+constexpr int kQMaxDepth = 64;
 constexpr int kQMaxLayers = 7;           // adjacency bit planes: an edge may be listed up to 96 times
 constexpr int kQSmallBits = 12;          // half registers of up to 2^12 amplitudes stay on chip
 constexpr int kQTile = 1 << kQSmallBits;
@@ -370,7 +371,7 @@ __device__ __forceinline__ void phase_table(double2* s_ph, int E, double gamma, 
 
 // An instance whose half register is streamed through tiles (m > 12).
 template <int TB>
-__device__ void qaoa_stream(const QaoaInst& I, const double* prm, double* grd, double* energy, const uint32_t* nb,
+__device__ void qaoa_stream(const QaoaInst& I, const double* prm, const Mix* mix, double* grd, double* energy, const uint32_t* nb,
                             double2* s_ph, double2* psi, double2* bufs, double2* red, bool with_grad) {
     const int n = I.n, p = I.p, E = I.n_edges, m = n - 1;
     double2* phi = psi + (1ull << m);
@@ -385,7 +386,7 @@ __device__ void qaoa_stream(const QaoaInst& I, const double* prm, double* grd, d
         w.up = k < p || with_grad;
         w.amp0 = 1.0;
         if (k < p) {
-            w.mu = mix_of(*QSV_DBG(prm + (2 * k + 1)), n);
+            w.mu = mix[k];
             phase_table(s_ph, E, *QSV_DBG(prm + 2 * k), k == 0 ? exp2(-0.5 * n) : prev.scn, false);
             prev = w.mu;
             qaoa_pass<TB, kForward>((k & 1) == 0, w, n, E, nb, I.layers, s_ph, psi, phi, bufs, acc);
@@ -409,7 +410,7 @@ __device__ void qaoa_stream(const QaoaInst& I, const double* prm, double* grd, d
         w.phase = w.up = r > 0;
         if (r > 0) {
             phase_table(s_ph, E, *QSV_DBG(prm + 2 * r), prev.scn, true);
-            w.mu = mix_of(*QSV_DBG(prm + (2 * r - 1)), n);
+            w.mu = mix[r - 1];
         }
         acc = PassSums{0, gb, 0, 0};
         qaoa_pass<TB, kReverse>(set_a, w, n, E, nb, I.layers, s_ph, psi, phi, bufs, acc);
@@ -425,7 +426,7 @@ __device__ void qaoa_stream(const QaoaInst& I, const double* prm, double* grd, d
 
 // An instance whose half register stays on chip (m <= 12): registers between layout changes, psi
 // in `A` and phi in `B` at them.  Index bits at and above m hold zeros.
-__device__ __noinline__ void qaoa_small(const QaoaInst& I, const double* prm, double* grd, double* energy, const uint32_t* nb, double2* s_ph,
+__device__ __noinline__ void qaoa_small(const QaoaInst& I, const double* prm, const Mix* mix, double* grd, double* energy, const uint32_t* nb, double2* s_ph,
                            double2* A, double2* B, double2* red, bool with_grad) {
     const int n = I.n, p = I.p, E = I.n_edges, m = n - 1;
     const uint32_t M = 1u << m, full = M - 1u, t = threadIdx.x;
@@ -436,7 +437,8 @@ __device__ __noinline__ void qaoa_small(const QaoaInst& I, const double* prm, do
         const int q[3] = {3 * g, 3 * g + 1, 3 * g + 2};
         cuts8(base_of(t, 3 * g), q, nb, I.layers, n, c);
     };
-    for (uint32_t i = t; i < kQTile; i += blockDim.x) A[i] = B[i] = make_double2(0.0, 0.0);
+    // the places that layouts 0..top reach
+    for (uint32_t i = t; i < (1u << (3 * (top + 1))); i += blockDim.x) A[i] = B[i] = make_double2(0.0, 0.0);
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
         v[s] = make_double2(base_of(t, 0) + s < M ? 1.0 : 0.0, 0.0);
@@ -510,7 +512,7 @@ __device__ __noinline__ void qaoa_small(const QaoaInst& I, const double* prm, do
 #pragma unroll
             for (int s = 0; s < 8; ++s) v[s] = cmul2(s_ph[c[s]], v[s]);
         }
-        prev = mix_of(*QSV_DBG(prm + (2 * r + 1)), n);
+        prev = mix[r];
         mixer(prev, std::false_type{}, none);
     }
     double e = 0.0;
@@ -548,7 +550,7 @@ __device__ __noinline__ void qaoa_small(const QaoaInst& I, const double* prm, do
             *QSV_DBG(grd + 2 * r) = 4.0 * sum.y;
             *QSV_DBG(grd + (2 * r + 1)) = 4.0 * sum.x;
         }
-        if (r > 0) prev = mix_of(*QSV_DBG(prm + (2 * r - 1)), n);
+        if (r > 0) prev = mix[r - 1];
     }
 }
 
@@ -565,6 +567,7 @@ __global__ void __launch_bounds__(kQThreads, 1)
     __shared__ uint32_t s_nb[32 * kQMaxLayers];
     __shared__ int s_ed[2 * kQMaxEdges];
     __shared__ double2 s_ph[kQMaxEdges + 1];
+    __shared__ Mix s_mix[kQMaxDepth];
     __shared__ double2 red[kQThreads / 32];
     for (;;) {
         __syncthreads();
@@ -577,7 +580,13 @@ __global__ void __launch_bounds__(kQThreads, 1)
         for (int u = threadIdx.x; u < 32 * kQMaxLayers; u += blockDim.x) s_nb[u] = 0;
         for (int e = threadIdx.x; e < 2 * I.n_edges; e += blockDim.x) s_ed[e] = *QSV_DBG(edges + (2 * I.edge_off + e));
         __syncthreads();
-        if (threadIdx.x == 0)     // adjacency with multiplicity: a ripple carry through the bit planes
+        if (threadIdx.x < 32 && I.layers == 1) {   // no edge twice: bits in any order
+            for (int e = threadIdx.x; e < I.n_edges; e += 32) {
+                const int a = s_ed[2 * e], b = s_ed[2 * e + 1];
+                atomicXor(&s_nb[a], 1u << b);
+                atomicXor(&s_nb[b], 1u << a);
+            }
+        } else if (threadIdx.x == 0) {   // adjacency with multiplicity: a ripple carry through the bit planes
             for (int e = 0; e < I.n_edges; ++e) {
                 const int a = s_ed[2 * e], b = s_ed[2 * e + 1];
                 for (int k = 0; k < kQMaxLayers; ++k) {
@@ -587,14 +596,20 @@ __global__ void __launch_bounds__(kQThreads, 1)
                     if (!carry) break;
                 }
             }
-        __syncthreads();
+        }
         const double* prm = params + I.param_off;
+        // Every layer's mixer angle, beside the first warp's adjacency: formed layer by layer they were half
+        // a microsecond of chain each, felt where the register is narrow (8 qubits, p = 4: 74 -> 68 us alone,
+        // 1000 of them 830 -> 795 us).
+        if (threadIdx.x >= 32)
+            for (int r = threadIdx.x - 32; r < I.p; r += blockDim.x - 32) s_mix[r] = mix_of(*QSV_DBG(prm + (2 * r + 1)), I.n);
+        __syncthreads();
         double* grd = grads + I.param_off;
         double* en = energy + id;
         double2* psi = pool + (I.state_off >= 0 ? I.state_off : static_cast<int64_t>(blockIdx.x) * cta_slot);
-        if (I.n - 1 <= kQSmallBits) qaoa_small(I, prm, grd, en, s_nb, s_ph, bufs, bufs + kQTile, red, with_grad != 0);
-        else if (I.n - 1 <= 21) qaoa_stream<11>(I, prm, grd, en, s_nb, s_ph, psi, bufs, red, with_grad != 0);
-        else qaoa_stream<12>(I, prm, grd, en, s_nb, s_ph, psi, bufs, red, with_grad != 0);
+        if (I.n - 1 <= kQSmallBits) qaoa_small(I, prm, s_mix, grd, en, s_nb, s_ph, bufs, bufs + kQTile, red, with_grad != 0);
+        else if (I.n - 1 <= 21) qaoa_stream<11>(I, prm, s_mix, grd, en, s_nb, s_ph, psi, bufs, red, with_grad != 0);
+        else qaoa_stream<12>(I, prm, s_mix, grd, en, s_nb, s_ph, psi, bufs, red, with_grad != 0);
     }
 }
 
@@ -673,7 +688,7 @@ void* qaoa_create(int device, int n_inst, const int32_t* n_qubits, const int32_t
         for (int i = 0; i < n_inst; ++i) {
             const int n = n_qubits[i], p = depth[i], E = edge_ptr[i + 1] - edge_ptr[i];
             if (n < 2 || n > kQMaxQubits) throw std::invalid_argument("QAOA instance width must be in [2, 24]");
-            if (p < 1 || p > 64) throw std::invalid_argument("QAOA depth must be in [1, 64]");
+            if (p < 1 || p > kQMaxDepth) throw std::invalid_argument("QAOA depth must be in [1, 64]");
             if (E < 0 || E > kQMaxEdges) throw std::invalid_argument("QAOA instance has too many edges");
             for (int e = edge_ptr[i]; e < edge_ptr[i + 1]; ++e) {
                 const int u = edges[2 * e], v = edges[2 * e + 1];
