@@ -1775,7 +1775,9 @@ bool run_adjoint_compiled(const std::vector<Op>& ops, double2* psi, double2* phi
     // a pass ends where its accumulators or its parameters would overflow (at most 32 doubles of phase
     // table and ratio a step, or the step's matrix)
     std::vector<TilePass> passes;
-    for (TilePass& p : plan_tiles(ops, n, kRtQubits, coalesced_low_qubits(16), kJitPlanSeeds)) {
+    // Seeded plans save a pass now and then and take the host 0.2 ms more for 400 steps: a pass takes that
+    // long from 24 qubits on (14 qubits, 3 layers: 601 -> 568 us without; 22 qubits, 8 layers 4.35 -> 4.14 ms).
+    for (TilePass& p : plan_tiles(ops, n, kRtQubits, coalesced_low_qubits(16), n < 24 ? 0 : kJitPlanSeeds)) {
         if (p.tile_qubits.empty()) {
             for (const Op& o : p.ops)
                 if (o.kind == OP_ADJ) return false;
