@@ -143,7 +143,7 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c
     return d;
 }
 
-template <int K, int C>
+template <int K, int C, bool EARLY = true>
 __global__ void __launch_bounds__(kThreads, (K <= 3 ? 4 : 3))   // 4 qubits: both pair sets stay in registers
     k_dense_reg_x2(float2* __restrict__ s, uint64_t n_groups, const __grid_constant__ DenseArgsX2<K> a) {
     constexpr int D = 1 << K;
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kThreads, (K <= 3 ? 4 : 3))   // 4 qubits: bot
     if (g >= n_groups) return;
     uint64_t base = insert_zeros(g, a.pos, K + C);
     if constexpr (C != 0) base |= a.ctrl;
-    after_predecessor();
+    if constexpr (EARLY) after_predecessor();
     uint64_t in[D], sw[D];
 #pragma unroll
     for (int l = 0; l < D; ++l) {
@@ -384,6 +384,16 @@ void launch_dense_reg(const Op& op, vec2_t<T>* s, int n, cudaStream_t st) {
         for (int e = 0; e < (1 << (2 * K)); ++e) {
             b.mr[e] = pack_f32x2(a.m[e].re, a.m[e].re);
             b.mi[e] = pack_f32x2(-a.m[e].im, a.m[e].im);
+        }
+        // One-qubit gates on a register of 32 or 64 MiB are blocks too short for the wait's own latency (24 of
+        // them: 22 qubits 222 us without it, 244 with, 23 qubits 368 and 450; below and above it gains:
+        // 21 qubits 170 and 141, 24 qubits 1060 and 1017).
+        if constexpr (K == 1) {
+            if (n == 22 || n == 23) {
+                const auto kern = nc ? k_dense_reg_x2<K, 1, false> : k_dense_reg_x2<K, 0, false>;
+                kern<<<static_cast<unsigned>(blocks), kThreads, 0, st>>>(s, groups, b);
+                return;
+            }
         }
         launch_early<float2*, uint64_t, DenseArgsX2<K>>(nc ? k_dense_reg_x2<K, 1> : k_dense_reg_x2<K, 0>, blocks, st, s,
                                                         groups, b);

@@ -782,3 +782,22 @@ def test_compiled_passes_fixed_matrices_change(dtype, tol, restatement):
         reg.close()
         err = float(np.max(np.abs(got - want)))
         assert err < tol, f"seed {s}: {err}"
+
+
+# complex64 one-qubit passes on both sides of and within the widths that launch them without overlap: 30
+# gates, each within 4 roundings of amplitudes that stay below 4 times 2^(-n/2)
+@pytest.mark.parametrize("n", [21, 22, 23, 24])
+def test_one_qubit_streams_in_both_storage_types(n):
+    from openqarp_b200.ir import ControlledUnitaryRecord
+    u = np.array([[0.6, 0.8j], [0.8j, 0.6]])
+    buf = ir.pack([Command(G.H, (q,)) for q in range(n)]
+                  + [x for q in (0, 1, 7, n - 2) for x in (Command(G.Rx, (q,), (0.4 + q,)),
+                                                           ControlledUnitaryRecord((q + 1,), q, u))]).buf
+    states = []
+    for dtype in ("complex64", "complex128"):
+        reg = Register(n, dtype)
+        reg.configure(0, 0, 0)
+        reg.apply(buf)
+        states.append(reg.get_state())
+        reg.close()
+    assert np.max(np.abs(states[0] - states[1])) < 40 * 4 * 2.0 ** -24 * 2.0 ** (-n / 2) * 4
