@@ -1278,9 +1278,6 @@ void cb_finalize(CircuitBatch* b) {
     check_cuda(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "batch stream");
     check_cuda(cudaEventCreate(&b->e0), "event");
     check_cuda(cudaEventCreate(&b->e1), "event");
-    check_cuda(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming), "event");
-    for (cudaEvent_t& e : b->join) check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-    for (cudaStream_t& t : b->side) check_cuda(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking), "batch stream");
     // every step reads its coefficients from the batch-wide table (encode appended each
     // instance's to it, so the offsets are absolute already): check that every read stays in it
     for (const FsStep& f : b->steps)
@@ -1352,6 +1349,7 @@ void cb_finalize(CircuitBatch* b) {
         c.i0 = at;
         while (at < n_inst && width_class(idev[at].n) == k) ++at;
         c.i1 = at;
+        if (c.i0 == c.i1) continue;
         const size_t smem = 2 * (size_t{1} << c.sm_qubits) * sizeof(double2);
         check_cuda(cudaFuncSetAttribute(c.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
                    "batch smem");
@@ -1360,6 +1358,14 @@ void cb_finalize(CircuitBatch* b) {
         int per_sm = 0;
         check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, c.kern, c.threads, smem), "occupancy");
         c.grid = static_cast<unsigned>(std::min<size_t>(c.i1 - c.i0, static_cast<size_t>(sms) * std::max(per_sm, 1)));
+    }
+    // the first class that has instances runs on the batch's own stream, each further one beside it
+    int branches = 0;
+    for (const Class& c : cls) branches += c.grid > 0;
+    if (branches > 1) check_cuda(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming), "event");
+    for (int k = 0; k + 1 < branches; ++k) {
+        check_cuda(cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming), "event");
+        check_cuda(cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking), "batch stream");
     }
     b->wide_qubits = 0;
     for (const CbInstHost& h : b->inst)
@@ -1373,11 +1379,11 @@ void cb_finalize(CircuitBatch* b) {
     check_cuda(cudaMemcpyAsync(b->dev + b->off_coef, b->host_coef, b->coef.size() * sizeof(double),
                                cudaMemcpyHostToDevice, b->stream), "batch coefficients");
     check_cuda(cudaMemsetAsync(b->dev + b->off_queue, 0, 3 * sizeof(int), b->stream), "batch queue");
-    check_cuda(cudaEventRecord(b->fork, b->stream), "batch fork");
-    for (int c = 0; c < 3; ++c) {
+    if (branches > 1) check_cuda(cudaEventRecord(b->fork, b->stream), "batch fork");
+    for (int c = 0, branch = 0; c < 3; ++c) {
         if (!cls[c].grid) continue;
-        cudaStream_t on = c == 0 ? b->stream : b->side[c - 1];
-        if (c) check_cuda(cudaStreamWaitEvent(on, b->fork, 0), "batch fork");
+        cudaStream_t on = branch == 0 ? b->stream : b->side[branch - 1];
+        if (branch) check_cuda(cudaStreamWaitEvent(on, b->fork, 0), "batch fork");
         cls[c].kern<<<cls[c].grid, cls[c].threads, 2 * (size_t{1} << cls[c].sm_qubits) * sizeof(double2), on>>>(
             reinterpret_cast<const CbInstDev*>(b->dev + b->off_inst), static_cast<int>(cls[c].i0),
             static_cast<int>(cls[c].i1), reinterpret_cast<const FsStep*>(b->dev + b->off_steps),
@@ -1387,10 +1393,11 @@ void cb_finalize(CircuitBatch* b) {
             reinterpret_cast<int*>(b->dev + b->off_queue) + c, reinterpret_cast<double*>(b->dev + b->off_energy),
             reinterpret_cast<double2*>(b->dev + b->off_slots), b->wide, b->wide_qubits, cls[c].sm_qubits);
         check_cuda(cudaGetLastError(), "batch launch");
-        if (c) {
-            check_cuda(cudaEventRecord(b->join[c - 1], on), "batch join");
-            check_cuda(cudaStreamWaitEvent(b->stream, b->join[c - 1], 0), "batch join");
+        if (branch) {
+            check_cuda(cudaEventRecord(b->join[branch - 1], on), "batch join");
+            check_cuda(cudaStreamWaitEvent(b->stream, b->join[branch - 1], 0), "batch join");
         }
+        ++branch;
     }
     check_cuda(cudaMemcpyAsync(b->host_out, b->dev + b->off_energy, n_inst * sizeof(double), cudaMemcpyDeviceToHost,
                                b->stream), "batch energies");
