@@ -170,11 +170,93 @@ def static_and_parities():
     reg.close()
 
 
+def compiled_sweeps():
+    """Circuits from |0...0> (tiles the circuit has not reached left out) and gradients in compiled
+    passes, one segment of which falls back to the interpreter."""
+    from openqarp_b200 import B200Simulator
+    n = 17
+    cmds = circuits.brickwork(n, 3, seed=8)
+    want = ORACLE.statevector(ir.pack(cmds).buf, n)
+    for dtype, tol in (("complex128", 1e-12), ("complex64", 1e-5)):
+        sim = B200Simulator(dtype=dtype)
+        sim.executor, sim.fusion_max_qubits = 3, 1
+        assert np.max(np.abs(sim.statevector(cmds, n) - want)) < tol, dtype
+        sim.close()
+    n = 15
+    cmds, vals, names = circuits.hea(n, 2, seed=3)
+    cmds.insert(50, ir.custom((3, 9, 0, 12), random_unitary(4, np.random.default_rng(4))))
+    stream = ir.pack(cmds, vals, names)
+    masks = observable.to_masks(circuits.tfim_chain(n), n)
+    e_or, g_or = ORACLE.adjoint(stream, n, len(names), masks)
+    reg = Register(n)
+    reg.configure(1, 0, 3)
+    reg.set_checkpoint_interval(40)
+    e, g = reg.adjoint(stream, len(names), masks)
+    reg.close()
+    assert abs(e - e_or) < 1e-10 and np.max(np.abs(np.asarray(g) - g_or)) < 1e-9
+
+
+def pauli_tiles():
+    """Energies whose partners lie in shared-memory tiles, against the kernel of two registers."""
+    n = 22
+    masks = observable.to_masks(circuits.tfim_chain(n) + circuits.random_pauli_sum(n, 40, seed=3, max_weight=4), n)
+    regs = [Register(n) for _ in range(2)]
+    for r in regs:
+        r.apply(ir.pack(circuits.brickwork(n, 2, seed=5)).buf)
+    assert abs(regs[0].expectation(masks) - regs[0].transition(regs[1], masks)) < 1e-10
+    for r in regs:
+        r.close()
+
+
+def streamed_qaoa():
+    """Batched QAOA on half registers streamed through both tile widths."""
+    from openqarp_b200.batch import QaoaBatch, QaoaInstance
+    rng = np.random.default_rng(6)
+    inst = [QaoaInstance(n, 2, [(q, (q + 1) % n) for q in range(n)]) for n in (14, 15, 23)]
+    params = [rng.uniform(0, np.pi, 4) for _ in inst]
+    q = QaoaBatch(inst)
+    e, g, _ = q.run(params)
+    q.close()
+    for k, (it, prm) in enumerate(zip(inst[:2], params)):
+        cmds, names, cost = circuits.qaoa_maxcut(it.n, it.edges, it.p)
+        e_or, g_or = ORACLE.adjoint(ir.pack(cmds, dict(zip(names, prm)), names), it.n, len(names),
+                                    observable.to_masks(cost, it.n))
+        assert abs(e[k] - e_or) < 1e-10 and np.max(np.abs(np.asarray(g[k]) - g_or)) < 1e-10, k
+
+
+def grouped_trajectories():
+    """Channels and measurements decided four qubits at a time (the lowest four among them) and segments
+    of CX and SWAP moved in one pass; the same seed gives the same outcomes whatever the batch."""
+    from openqarp_b200.noise import NoiseModel
+    n = 14
+    cmds = []
+    for layer in range(2):
+        cmds += [Command(G.Ry, (q,), (0.3 + q + layer,)) for q in range(n)]
+        cmds += [Command(G.CX, (q, q + 1)) for q in range(n - 1)] + [Command(G.SWAP, (layer, n - 1))]
+        cmds.append(Command(G.Measure, (layer,), (), None, (layer,)))
+    cmds += [Command(G.Measure, (q,), (), None, (q,)) for q in range(n)]
+    buf = ir.pack(cmds).buf
+    for dtype in ("complex128", "complex64"):
+        for noisy in (False, True):
+            runs = []
+            for batch in (64, 16):
+                reg = Register(n, dtype)
+                reg.configure(1, 0)
+                reg.set_trajectory_batch(batch)
+                if noisy:
+                    reg.set_noise(NoiseModel.amplitude_damping(0.1, ["Ry"]))
+                runs.append(reg.run_trajectories(buf, 3, 64)[:2])
+                reg.close()
+            assert np.array_equal(runs[0][0], runs[1][0]) and np.array_equal(runs[0][1], runs[1][1]), (dtype, noisy)
+
+
 if __name__ == "__main__":
     for name, fn in (("self-test", selftest), ("executors", executors),
                      ("reductions and sampling", reductions_and_sampling), ("adjoint", adjoint),
                      ("batches", batches), ("trajectories", trajectories),
-                     ("static transition and parities", static_and_parities)):
+                     ("static transition and parities", static_and_parities),
+                     ("compiled sweeps", compiled_sweeps), ("Pauli tiles", pauli_tiles),
+                     ("streamed QAOA", streamed_qaoa), ("grouped trajectories", grouped_trajectories)):
         fn()
         print(f"ok {name}", flush=True)
     print("ALL OK", flush=True)
