@@ -350,8 +350,6 @@ struct KrausPass {
     int32_t n_sum;                 // how many (0: no sums)
 };
 
-// Group index g names the amplitudes that differ in the MA applied qubits; bits 0..4 of g are the
-// lane, 5..7 the warp, then the thread's iterations and the block.
 // Where the block's amplitude i lies when qubits 0..3 are the ones applied (LOW): a thread's 16 are
 // consecutive then, and the place in a 128-byte row is XORed so that 8 (16) lanes cover all banks.
 template <typename T>
@@ -359,6 +357,8 @@ __device__ __forceinline__ uint32_t low_place(uint32_t i) {
     return i ^ ((i >> 4) & (sizeof(T) == 8 ? 7u : 15u));
 }
 
+// Group index g names the amplitudes that differ in the MA applied qubits; bits 0..4 of g are the
+// lane, 5..7 the warp, then the thread's iterations and the block.
 // LOW: the applied qubits are 0..3, so a lane's amplitudes would be 256 bytes from the next lane's
 // (715 us at 26 qubits against 441 for higher qubits): the block's 4096 amplitudes go through shared
 // memory instead, read and written in order (498 us).

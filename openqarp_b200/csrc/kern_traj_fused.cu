@@ -302,7 +302,7 @@ struct FsShot {
 };
 
 // A step costs a chain of a few hundred cycles (record, indices, the unit's latency, a barrier),
-// shared-memory traffic second.  10 qubits, 20000 shots of about 80 steps: 8.54 ms with 64-bit
+// shared-memory traffic second.  10 qubits, 20000 shots of about 140 steps: 8.54 ms with 64-bit
 // indices, rows one at a time, whole engines seeded and twisted and 256 threads a shot; 4.9 ms now.
 //
 // Shots of NT threads, W of them to a block.  W > 1 is a shot per warp (NT = 32, resident plan): a

@@ -208,9 +208,10 @@ std::vector<Op> lower(const Cmd& c, int n) {
             return {make_dense1(c.q[0], fixed(g))};
         case RX: return {make_dense1(c.q[0], m_rx(param(c, 0)))};
         case RY: {
-            Op o = make_dense1(c.q[0], m_ry(param(c, 0)));
-            o.y_turn = true;
-            return {o};
+            std::vector<Op> ops;
+            ops.push_back(make_dense1(c.q[0], m_ry(param(c, 0))));
+            ops[0].y_turn = true;
+            return ops;
         }
         case U: return {make_dense1(c.q[0], m_u(param(c, 0), param(c, 1), param(c, 2)))};
         case Z: case S: case SDG: case T: case TDG:
