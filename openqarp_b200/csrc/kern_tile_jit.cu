@@ -257,7 +257,7 @@ struct Gen {
 
     // Coefficients come in pairs, real ones with a 0 beside them: a complex entry that straddles 16
     // bytes is read in halves, and ptxas then spills amplitudes (28-qubit brickwork in complex128: 2680
-    // bytes of spill stores over its 15 passes against 1150, 48.7 against 47.1 ms; 600 as it is now).
+    // bytes of spill stores over its 15 passes against 1150, 48.7 against 47.1 ms; 656 as it is now).
     size_t push(c128 v) {
         coef.push_back(v.real());
         coef.push_back(v.imag());
@@ -1131,9 +1131,6 @@ constexpr bool kJitDebug = true;
 const char* kPreludeDebug = "";
 constexpr bool kJitDebug = false;
 #endif
-// Complex128 stores walk a pointer by JitStore::step; complex64 ones, and the debug build's checked
-// ones, take an index each (pass_source).
-bool jit_walks(bool f32) { return !kJitDebug && !f32; }
 static_assert(kRtRegBits == 4, "JitStore::step and the kernels' d0..d3");
 
 // Walk one pass's plan: coefficients, structural signature and (with emit) the steps' source.
@@ -1297,38 +1294,20 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
     const int chunks = (1 << kRtQubits) >> low;
     std::string gtid = "0ull";
     for (int b = 0; b < 8; ++b)
-        gtid += " | ((u64)((ct >> " + std::to_string(b) + ") & 1u) << " + std::to_string(tq[b + low]) + ")";
+        gtid += " | ((u64)((tid >> " + std::to_string(b) + ") & 1u) << " + std::to_string(tq[b + low]) + ")";
     // store: the last layout's lanes are local bits 0..4
     std::string gfin = "0ull";
     for (int k = 0; k < kRtLaneBits; ++k)
-        gfin += " | ((u64)((ft >> " + std::to_string(k) + ") & 1u) << " + std::to_string(tq[F.lane[k]]) + ")";
+        gfin += " | ((u64)((lane >> " + std::to_string(k) + ") & 1u) << " + std::to_string(tq[F.lane[k]]) + ")";
     for (int k = 0; k < kRtWarpBits; ++k)
-        gfin += " | ((u64)((ft >> " + std::to_string(kRtLaneBits + k) + ") & 1u) << " + std::to_string(tq[F.warp[k]]) + ")";
+        gfin += " | ((u64)((warp >> " + std::to_string(k) + ") & 1u) << " + std::to_string(tq[F.warp[k]]) + ")";
     // a global amplitude index: checked against the register in the debug build
     const std::string dim = hex64(1ull << n);
     auto at = [&](const std::string& e) {
         return kJitDebug ? "dbg_idx(" + e + ", " + dim + ", dbg)" : "(" + e + ")";
     };
-    // Thread offsets are formed where a tile is asked for (ct) and where it is stored (ft), from opaque
-    // copies of the thread number where keeping them through the steps costs amplitudes' registers (else
-    // the compiler keeps them).  Complex128, 26 qubits, three-qubit blocks: 9.98 -> 9.60 ms.  Complex64:
-    // only what a tile is asked by, and only in passes with Pauli rotations (30-qubit Heisenberg step 18.04
-    // -> 17.76 ms; the 28-qubit brickwork, which has none, 25.85 -> 27.2).  Pair passes have registers to
-    // spare: neither, and they form the store's strides themselves (24 qubits, 8 layers: 10.94 against
-    // 11.20 ms).
-    const bool paulis = std::any_of(plan.steps.begin(), plan.steps.end(), [](const RtStep& st) { return st.kind == RT_PAULI; });
-    auto opaque = [](const char* v, bool on) {
-        return on ? std::string("    asm volatile(\"\" : \"+r\"(") + v + "));\n" : std::string();
-    };
-    std::string strides;
-    for (int p = 0; p < kRtRegBits && pair && jit_walks(f32); ++p) {
-        const std::string q = std::to_string(tq[F.reg[p]]);
-        strides += "  const long long d" + std::to_string(p) + " = (turned >> " + q + ") & 1 ? -(1ll << " + q + ") : 1ll << " + q + ";\n";
-    }
     auto issue = [&](const std::string& b) {
         std::ostringstream x;
-        x << "    unsigned ct = threadIdx.x;\n" << opaque("ct", !pair && (!f32 || paulis)) << "    const u64 gtid = " << gtid
-          << ";\n    const unsigned stid = swz(ct);\n";
         for (int j = 0; j < chunks / kJitThreads; ++j) {
             uint64_t gj = 0;
             for (int b2 = 0; b2 < 4 && 8 + low + b2 < kRtQubits; ++b2)
@@ -1346,10 +1325,10 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
     } else {
         s << "typedef double R; typedef double2 R2;\n#define FMA fma\n#define MK make_double2\n";
     }
-    s << "struct __align__(16) C" << idx << " { R c[" << nc << "]; };\n"
+    s << "struct __align__(8) C" << idx << " { R c[" << nc << "]; };\n"
       << "extern \"C\" __global__ void __launch_bounds__(" << kJitThreads << ", " << (pair ? 1 : jit_ctas(f32))
       << ") qsv_jit_" << idx << "(R2* __restrict__ s, unsigned n_tiles, unsigned tmask, unsigned tstep, u64 turned, "
-      << (jit_walks(f32) && !pair ? "long long d0, long long d1, long long d2, long long d3, " : "")
+      << (kJitDebug ? "" : "long long d0, long long d1, long long d2, long long d3, ")
       << (pair ? "R2* __restrict__ s2, double2* __restrict__ partials, " : "") << "const __grid_constant__ C" << idx << " P"
       << (kJitDebug ? ", unsigned long long* __restrict__ dbg" : "") << ") {\n"
       << "  extern __shared__ __align__(16) unsigned char smem[];\n"
@@ -1360,10 +1339,12 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
           << (1 << kRtQubits) << ");\n  for (unsigned k = 0; k < " << n_acc << "u; ++k) acc[k * " << kJitThreads
           << "u + threadIdx.x] = 0;\n";
     s << "  const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;\n"
+      << "  const u64 gtid = " << gtid << ";\n"
+      << "  const unsigned stid = swz(tid);\n"
+      << "  const u64 gfin = " << gfin << ";\n"
       // the i-th tile is the i-th subset of tmask; tstep = spread(gridDim.x, tmask), added with the
       // carries running through the other bits
       << "  unsigned i = blockIdx.x, t = spread(i, tmask);\n"
-      << strides
       << "  if (i < n_tiles) {\n    const u64 b0 = " << deposit("t") << ";\n" << issue("b0") << "  }\n"
       << "  asm volatile(\"cp.async.commit_group;\\n\" ::: \"memory\");\n"
       << "  for (; i < n_tiles; i += gridDim.x, t = ((t | ~tmask) + tstep) & tmask) {\n"
@@ -1394,9 +1375,8 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
       << "  if (i + gridDim.x < n_tiles) {\n    const unsigned tn = ((t | ~tmask) + tstep) & tmask;\n    const u64 b1 = " << deposit("tn")
       << ";\n" << issue("b1") << "  }\n"
       << "  asm volatile(\"cp.async.commit_group;\\n\" ::: \"memory\");\n";
-    s << "  unsigned ft = threadIdx.x;\n" << opaque("ft", !pair && !f32)
-      << "  const u64 to = (base | " << gfin << ") ^ turned;\n";
-    for (int r = 0; r < kJitAmps && !jit_walks(f32); ++r) {
+    s << "  const u64 to = (base | gfin) ^ turned;\n";
+    for (int r = 0; kJitDebug && r < kJitAmps; ++r) {
         uint64_t gc = 0;
         for (int p = 0; p < kRtRegBits; ++p)
             if ((r >> p) & 1) gc |= 1ull << tq[F.reg[p]];
@@ -1404,12 +1384,12 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
             s << "  __stcs(" << (set == 'a' ? "s" : "s2") << " + " << at("to ^ " + hex64(gc)) << ", MK(" << re(set, r) << ", "
               << im(set, r) << "));\n";
     }
-    // The slots in Gray order, a pointer stepping by a slot bit's stride, negative where the bit is turned.
-    // The strides are kernel parameters and tile numbers 32-bit: formed in the kernel and 64-bit they
-    // took the registers that the amplitudes need (28 qubits, depth 20, complex128: 47.1 -> 46.3 ms
-    // applied again and again; an XOR and a scaled address per store 46.3 too, but 13.0 against 12.7 ms
-    // with two-qubit blocks at 26 qubits; complex64: XOR 25.6, pointer 25.9).
-    if (jit_walks(f32)) {
+    // The slots in Gray order, a pointer stepping by a slot bit's stride, negative where the bit is turned
+    // (the debug build checks an index per store instead).  The strides are kernel parameters and tile
+    // numbers 32-bit: formed in the kernel and 64-bit they took the registers that the amplitudes need
+    // (28 qubits, depth 20, complex128: 47.1 -> 46.3 ms applied again and again; an XOR and a scaled
+    // address per store 47.3).
+    if (!kJitDebug) {
         for (char set : sets) s << "  R2* w" << set << " = " << (set == 'a' ? "s" : "s2") << " + to;\n";
         for (int k = 0, r = 0; k < kJitAmps; ++k) {
             for (char set : sets) s << "  __stcs(w" << set << ", MK(" << re(set, r) << ", " << im(set, r) << "));\n";
@@ -1675,7 +1655,6 @@ JitPlan jit_prepare(const std::vector<const TilePass*>& passes, int n, int devic
             arg.assign(reinterpret_cast<const uint8_t*>(w.coef.data()),
                        reinterpret_cast<const uint8_t*>(w.coef.data() + w.coef.size()));
         }
-        arg.resize((arg.size() + 15) & ~size_t{15});     // the parameter struct's size
         out.coef.push_back(std::move(arg));
     }
     if (sigs.empty()) return out;
@@ -1764,7 +1743,7 @@ void launch_pass(const JitPlan& plan, int pass, void* s, void* s2, double2* part
         if (i & 1) tstep |= m & (0 - m);
     double2* part = partials ? partials + static_cast<size_t>(plan.acc0[static_cast<size_t>(k)]) * grid : nullptr;
     std::vector<void*> args{&s, &n_tiles, &tmask, &tstep, &store.turned};
-    if (jit_walks(plan.f32) && !plan.pair)
+    if (!kJitDebug)
         for (long long& d : store.step) args.push_back(&d);
     if (plan.pair) args.insert(args.end(), {static_cast<void*>(&s2), static_cast<void*>(&part)});
     args.push_back(const_cast<uint8_t*>(c.data()));
