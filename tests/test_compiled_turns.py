@@ -87,3 +87,32 @@ def test_coefficients_come_in_pairs(dtype, tmp_path, monkeypatch):
     assert len(singles) > 20 and len(products) > 100
     assert all(int(a or b) % 2 == 0 for a, b in singles)
     assert all(int(a) % 2 == 0 and int(b) == int(a) + 1 for a, b in products)
+
+
+# a pass of three-qubit blocks, a controlled one-qubit gate and a bit put back, whose amplitudes do not
+# all stay in registers, against the executor of single passes: a dozen products of unit-norm amplitudes
+@pytest.mark.gpu
+@pytest.mark.parametrize("seed", [1, 2])
+def test_pass_that_spills_amplitudes(seed):
+    from openqarp_b200.ir import ControlledUnitaryRecord, PermutationRecord
+    rng = np.random.default_rng(seed)
+
+    def unitary(k):
+        return np.linalg.qr(rng.standard_normal((1 << k, 1 << k)) + 1j * rng.standard_normal((1 << k, 1 << k)))[0]
+    n = 12
+    cmds = [Command(G.CH, (2, 11)), ir.custom((9, 7, 11, 10, 2), unitary(5)),
+            PermutationRecord((8, 4, 11), rng.permutation(8).astype(np.uint64)), Command(G.Rz, (9,), (np.pi,)),
+            Command(G.U, (7,), (1.2, 2.6, -np.pi)), ir.custom((1, 9, 5), unitary(3)), Command(G.Rx, (8,), (2 * np.pi,)),
+            Command(G.CRz, (1, 8), (4.54,)), ir.custom((4,), unitary(1)), Command(G.iSWAP, (6, 7)),
+            ControlledUnitaryRecord((5, 6, 9, 3), 7, unitary(4)), Command(G.Rx, (10,), (np.pi / 2,))]
+    start = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    start /= np.linalg.norm(start)
+    states = []
+    for executor in (3, 0):
+        reg = Register(n)
+        reg.configure(1, 0, executor)
+        reg.set_state(start)
+        reg.apply(ir.pack(cmds).buf)
+        states.append(reg.get_state())
+        reg.close()
+    assert np.max(np.abs(states[0] - states[1])) < 1e-13
