@@ -255,13 +255,19 @@ struct Gen {
     int normalised = 0;   // normalised tables since cglob was last applied
     double flops = 0;   // FP64 operations per thread per tile (FMA = 2, MUL = 1)
 
-    // Coefficients come in pairs, real ones with a 0 beside them: a complex entry that straddles 16
-    // bytes is read in halves, and ptxas then spills amplitudes (28-qubit brickwork in complex128: 2680
-    // bytes of spill stores over its 15 passes against 1150, 48.7 against 47.1 ms; 656 as it is now).
     size_t push(c128 v) {
         coef.push_back(v.real());
         coef.push_back(v.imag());
         return coef.size() - 2;
+    }
+    // A real coefficient.  Complex128: a pair with a 0, or the complex entries after it straddle 16 bytes,
+    // are read in halves, and ptxas spills amplitudes (28-qubit brickwork: 2680 bytes of spill stores over
+    // its 15 passes against 1150, 48.7 against 47.1 ms; 656 as it is now).  Complex64 takes single ones
+    // and 64-bit tile numbers: the 30-qubit Heisenberg step 17.87 ms, 18.04 to 18.24 in the other forms.
+    size_t real(double v) {
+        if (!f32) return push(v);
+        coef.push_back(v);
+        return coef.size() - 1;
     }
     static std::string cr(size_t at) { return "P.c[" + std::to_string(at) + "]"; }
     static std::string ci(size_t at) { return "P.c[" + std::to_string(at + 1) + "]"; }
@@ -512,7 +518,7 @@ struct Gen {
     void rotate(int p, int b, double c, double s, c128 d0, c128 d1) {
         const bool cos_form = std::abs(c) >= std::abs(s);
         double scale = cos_form ? c : s;
-        const size_t at = push(cos_form ? s / c : -(c / s));
+        const size_t at = real(cos_form ? s / c : -(c / s));
         if (pair) {
             cglob *= scale;
             scale = 1.0;
@@ -552,7 +558,7 @@ struct Gen {
     // form the host cannot rewrite.
     void unturn_slot(const RtLayout& L, int p) {
         const int b = L.reg[p];
-        const size_t at = push(turned[b] ? 1.0 : 0.0);
+        const size_t at = real(turned[b] ? 1.0 : 0.0);
         if (turned[b]) std::swap(pend[b][0], pend[b][1]);
         turned[b] = false;
         mark(0xF7u, static_cast<uint64_t>(p));
@@ -696,7 +702,7 @@ struct Gen {
                 *rm |= 1u << k;
                 continue;
             }
-            const size_t at = push(turned[b] ? 1.0 : 0.0);
+            const size_t at = real(turned[b] ? 1.0 : 0.0);
             c += (c.empty() ? "" : " && ") + std::string(w == 'l' ? "((((lane >> " : "((((warp >> ") + std::to_string(k) +
                  ") & 1u) != 0u) != (" + cr(at) + " != 0))";
         }
@@ -1105,8 +1111,9 @@ __device__ __forceinline__ double flip(double a, int m) {
 }
 __device__ __forceinline__ float flip(float a, int m) { return __int_as_float(__float_as_int(a) ^ m); }
 // the bits of i placed at the set bits of m, lowest first
-__device__ __forceinline__ unsigned spread(unsigned i, unsigned m) {
-    unsigned r = 0;
+template <typename U>
+__device__ __forceinline__ U spread(U i, U m) {
+    U r = 0;
     for (; i && m; i >>= 1, m &= m - 1)
         if (i & 1) r |= m & (0 - m);
     return r;
@@ -1131,6 +1138,9 @@ constexpr bool kJitDebug = true;
 const char* kPreludeDebug = "";
 constexpr bool kJitDebug = false;
 #endif
+// Complex128 stores walk a pointer by JitStore::step; complex64 ones, and the debug build's checked ones,
+// take an index each (pass_source).
+bool jit_walks(bool f32) { return !kJitDebug && !f32; }
 static_assert(kRtRegBits == 4, "JitStore::step and the kernels' d0..d3");
 
 // Walk one pass's plan: coefficients, structural signature and (with emit) the steps' source.
@@ -1318,6 +1328,7 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
         }
         return x.str();
     };
+    const std::string ix = f32 ? "u64" : "unsigned";      // tile numbers
     std::ostringstream s;
     if (f32) {
         s << "typedef float R; typedef float2 R2;\n#define FMA fmaf\n#define MK make_float2\n";
@@ -1327,8 +1338,8 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
     }
     s << "struct __align__(8) C" << idx << " { R c[" << nc << "]; };\n"
       << "extern \"C\" __global__ void __launch_bounds__(" << kJitThreads << ", " << (pair ? 1 : jit_ctas(f32))
-      << ") qsv_jit_" << idx << "(R2* __restrict__ s, unsigned n_tiles, unsigned tmask, unsigned tstep, u64 turned, "
-      << (kJitDebug ? "" : "long long d0, long long d1, long long d2, long long d3, ")
+      << ") qsv_jit_" << idx << "(R2* __restrict__ s, " << ix << " n_tiles, " << ix << " tmask, " << ix << " tstep, u64 turned, "
+      << (jit_walks(f32) ? "long long d0, long long d1, long long d2, long long d3, " : "")
       << (pair ? "R2* __restrict__ s2, double2* __restrict__ partials, " : "") << "const __grid_constant__ C" << idx << " P"
       << (kJitDebug ? ", unsigned long long* __restrict__ dbg" : "") << ") {\n"
       << "  extern __shared__ __align__(16) unsigned char smem[];\n"
@@ -1344,7 +1355,7 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
       << "  const u64 gfin = " << gfin << ";\n"
       // the i-th tile is the i-th subset of tmask; tstep = spread(gridDim.x, tmask), added with the
       // carries running through the other bits
-      << "  unsigned i = blockIdx.x, t = spread(i, tmask);\n"
+      << "  " << ix << " i = blockIdx.x, t = spread(i, tmask);\n"
       << "  if (i < n_tiles) {\n    const u64 b0 = " << deposit("t") << ";\n" << issue("b0") << "  }\n"
       << "  asm volatile(\"cp.async.commit_group;\\n\" ::: \"memory\");\n"
       << "  for (; i < n_tiles; i += gridDim.x, t = ((t | ~tmask) + tstep) & tmask) {\n"
@@ -1372,11 +1383,11 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
     s << "  }\n  __syncthreads();\n"
       << steps
       << "  __syncthreads();\n"
-      << "  if (i + gridDim.x < n_tiles) {\n    const unsigned tn = ((t | ~tmask) + tstep) & tmask;\n    const u64 b1 = " << deposit("tn")
+      << "  if (i + gridDim.x < n_tiles) {\n    const " << ix << " tn = ((t | ~tmask) + tstep) & tmask;\n    const u64 b1 = " << deposit("tn")
       << ";\n" << issue("b1") << "  }\n"
       << "  asm volatile(\"cp.async.commit_group;\\n\" ::: \"memory\");\n";
     s << "  const u64 to = (base | gfin) ^ turned;\n";
-    for (int r = 0; kJitDebug && r < kJitAmps; ++r) {
+    for (int r = 0; r < kJitAmps && !jit_walks(f32); ++r) {
         uint64_t gc = 0;
         for (int p = 0; p < kRtRegBits; ++p)
             if ((r >> p) & 1) gc |= 1ull << tq[F.reg[p]];
@@ -1384,12 +1395,11 @@ std::string pass_source(const TilePass& pass, const RtPlan& plan, int n, int idx
             s << "  __stcs(" << (set == 'a' ? "s" : "s2") << " + " << at("to ^ " + hex64(gc)) << ", MK(" << re(set, r) << ", "
               << im(set, r) << "));\n";
     }
-    // The slots in Gray order, a pointer stepping by a slot bit's stride, negative where the bit is turned
-    // (the debug build checks an index per store instead).  The strides are kernel parameters and tile
-    // numbers 32-bit: formed in the kernel and 64-bit they took the registers that the amplitudes need
-    // (28 qubits, depth 20, complex128: 47.1 -> 46.3 ms applied again and again; an XOR and a scaled
-    // address per store 47.3).
-    if (!kJitDebug) {
+    // The slots in Gray order, a pointer stepping by a slot bit's stride, negative where the bit is turned.
+    // The strides are kernel parameters and tile numbers 32-bit: formed in the kernel and 64-bit they
+    // took the registers that the amplitudes need (28 qubits, depth 20, complex128: 47.1 -> 46.3 ms
+    // applied again and again; an XOR and a scaled address per store 47.3).
+    if (jit_walks(f32)) {
         for (char set : sets) s << "  R2* w" << set << " = " << (set == 'a' ? "s" : "s2") << " + to;\n";
         for (int k = 0, r = 0; k < kJitAmps; ++k) {
             for (char set : sets) s << "  __stcs(w" << set << ", MK(" << re(set, r) << ", " << im(set, r) << "));\n";
@@ -1730,20 +1740,20 @@ void launch_pass(const JitPlan& plan, int pass, void* s, void* s2, double2* part
     check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "sm count");
     // tile numbers take n - 12 bits
     static_assert(QSV_MAX_QUBITS - kRtQubits < 32, "tile numbers are 32-bit in the kernels");
-    unsigned tmask = static_cast<unsigned>(tiles & ((1ull << (n - kRtQubits)) - 1));
-    unsigned n_tiles = 1u << __builtin_popcount(tmask);
+    unsigned long long tmask = tiles & ((1ull << (n - kRtQubits)) - 1);    // a 32-bit parameter takes the low half
+    unsigned long long n_tiles = 1ull << __builtin_popcountll(tmask);
     // a pair pass writes its partials by block: the grid its caller sized them for
     const unsigned grid = plan.pair ? adjoint_tile_grid(n, kRtQubits)
                                     : static_cast<unsigned>(std::min<uint64_t>(
                                           n_tiles, static_cast<uint64_t>(jit_ctas(plan.f32)) * static_cast<uint64_t>(sms)));
     const std::vector<uint8_t>& c = plan.coef[static_cast<size_t>(k)];
     JitStore store = plan.store[static_cast<size_t>(k)];
-    unsigned tstep = 0;      // spread(grid, tmask)
-    for (unsigned i = grid, m = tmask; i && m; i >>= 1, m &= m - 1)
+    unsigned long long tstep = 0;      // spread(grid, tmask)
+    for (unsigned long long i = grid, m = tmask; i && m; i >>= 1, m &= m - 1)
         if (i & 1) tstep |= m & (0 - m);
     double2* part = partials ? partials + static_cast<size_t>(plan.acc0[static_cast<size_t>(k)]) * grid : nullptr;
     std::vector<void*> args{&s, &n_tiles, &tmask, &tstep, &store.turned};
-    if (!kJitDebug)
+    if (jit_walks(plan.f32))
         for (long long& d : store.step) args.push_back(&d);
     if (plan.pair) args.insert(args.end(), {static_cast<void*>(&s2), static_cast<void*>(&part)});
     args.push_back(const_cast<uint8_t*>(c.data()));

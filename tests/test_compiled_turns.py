@@ -70,8 +70,8 @@ def test_diagonals_of_any_modulus(restatement, d, dtype, tol):
         reg.close()
 
 
-# what every pass reads of its coefficients is a whole pair (no device needed: the source is looked at)
-@pytest.mark.parametrize("dtype", [0, 1])
+# what a complex128 pass reads of its coefficients is a whole pair (no device needed: the source is looked at)
+@pytest.mark.parametrize("dtype", [0])
 def test_coefficients_come_in_pairs(dtype, tmp_path, monkeypatch):
     import ctypes
     import re
